@@ -8,11 +8,12 @@
 //
 // One thread per leaf: a warp reads 32 consecutive rows of a column as one
 // 128-byte transaction; the message schedule and state stay in registers.
-// Each CTA hashes 256 leaves and then folds the three node levels whose parents
-// fill whole warps (128, 64, 32) in shared memory, writing every level; a tree
-// that fits one CTA is folded to its root there. The layers above are folded by
-// k_merkle_nodes: four levels per launch while there are more than 2^12
-// children, then up to 9 levels per launch.
+// Each CTA hashes 256 leaves and then folds the three node levels whose parents fill whole warps
+// (128, 64, 32) in shared memory, writing every level; a tree that fits one CTA is folded to its root there. The layers above are
+// folded by k_merkle_nodes, four levels per launch, while there are more than 2^12 children, and the
+// rest by one launch of k_merkle_top.
+#include <cooperative_groups.h>
+
 #include <utility>
 
 #include "blake2s.cuh"
@@ -23,11 +24,13 @@ namespace sb {
 
 namespace {
 
+namespace cg = cooperative_groups;
+
 constexpr uint32_t LEAF_THREADS = 256;  // leaves per CTA
-constexpr uint32_t LEAF_LEVELS = 8;     // node levels folded inside a leaf CTA
+constexpr uint32_t LEAF_LEVELS = 8;     // a tree of up to 2^8 leaves folds in its leaf CTA
 constexpr uint32_t FULL_WARP_LEVELS = 3;  // levels whose parents fill whole warps (128, 64, 32)
 constexpr uint32_t NODE_THREADS = 256;  // parents per CTA at the first level
-constexpr uint32_t NODE_FOLD_LOG = 12;  // layers up to 2^12 nodes fold inside CTAs
+constexpr uint32_t NODE_FOLD_LOG = 12;  // layers of up to 2^12 nodes fold in one launch (k_merkle_top)
 
 struct Seeds { uint32_t leaf[8], node[8]; };
 
@@ -55,6 +58,27 @@ cudaError_t launch_chained(void (*kernel)(K...), dim3 grid, dim3 block, size_t s
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
+// The same for a grid that is one cluster of `ctas` CTAs.
+template <typename... K, typename... A>
+cudaError_t launch_cluster_chained(void (*kernel)(K...), uint32_t ctas, dim3 block, size_t smem, cudaStream_t stream,
+                                   A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = ctas;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = ctas;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
@@ -220,6 +244,190 @@ __global__ void __launch_bounds__(NODE_THREADS) k_merkle_nodes(uint8_t* layers, 
   fold_levels(sm, per_cta, levels, layers, max_log, child_log, first, seeds.node, one);
 }
 
+// ---- Node levels with few parents: four lanes per hash -------------------------------------------
+// A level of a few hashes is bound by the latency of one compression, and a warp that runs a whole
+// hash per lane issues all 1130 instructions of it (1.4 us, measured on levels of 32 parents or
+// fewer). Four lanes per hash, lane q holding column q of the state (v[q], v[4+q], v[8+q], v[12+q]),
+// issue one G step each per half round; between the column and the diagonal steps a, c and d move to
+// the neighbour lanes and b, the last word a G step completes, stays, so the shuffles hide behind the
+// steps around them. About 1.0 us a level. It takes 1.4 times
+// the instructions per hash, so levels of more than 128 parents per CTA, which keep a multiprocessor
+// busy, stay with one lane per hash. (The rounds as a loop, with the offsets in shared memory, took
+// 1.65 us a level: the loads and the loop lengthen the chain.)
+constexpr uint32_t QUAD_THREADS = 512;
+constexpr uint32_t QCAP = 512;             // hashes per buffer
+constexpr uint32_t QS = QCAP + 8;          // word stride: word w of hash i at w * QS + i; 8 extra words
+                                           // put the four lanes of a hash on different banks
+struct QuadBuffers { uint32_t w[2][8 * QS]; };
+
+__device__ __forceinline__ void put_hash(uint32_t* buf, uint32_t i, const uint32_t h[8]) {
+#pragma unroll
+  for (int w = 0; w < 8; ++w) buf[w * QS + i] = h[w];
+}
+
+// Message schedule (RFC 7693 section 2.7), one row a round, nibble j = the word of G-step operand j.
+__device__ __forceinline__ constexpr uint64_t b2s_sigma(int r) {
+  constexpr uint64_t rows[10] = {0xfedcba9876543210ull, 0x357b20c16df984aeull, 0x491763eadf250c8bull,
+                                 0x8f04a562ebcd1397ull, 0xd386cb1efa427509ull, 0x91ef57d438b0a6c2ull,
+                                 0xb8293670a4def15cull, 0xa2684f05931ce7bdull, 0x5a417d2c803b9ef6ull,
+                                 0x0dc3e9bf5167482aull};
+  return rows[r];
+}
+
+struct QuadLane {
+  uint32_t q, up1, up2, up3;  // this lane's column, and the lanes 1, 2 and 3 columns on
+  uint32_t iv, iv4;           // words q and 4 + q of the initial value
+  uint32_t ad[40];            // byte offsets of the 40 message words of this lane's G steps
+};
+
+__device__ __forceinline__ void quad_lane_init(QuadLane& L) {
+  const uint32_t q = threadIdx.x & 3, g = threadIdx.x >> 2;
+  L.q = q; L.up1 = (q + 1) & 3; L.up2 = (q + 2) & 3; L.up3 = (q + 3) & 3;
+  L.iv = q == 0 ? B2sIv::v0 : q == 1 ? B2sIv::v1 : q == 2 ? B2sIv::v2 : B2sIv::v3;
+  L.iv4 = q == 0 ? B2sIv::v4 : q == 1 ? B2sIv::v5 : q == 2 ? B2sIv::v6 : B2sIv::v7;
+  // Word k < 8 of a parent's message is word k of its left child 2g, k >= 8 word k - 8 of 2g + 1.
+  auto off = [&](uint32_t k) { return ((k & 7) * QS + (k >> 3) + 2 * g) * 4; };
+#pragma unroll
+  for (int r = 0; r < 10; ++r) {
+    const uint32_t col = (uint32_t)b2s_sigma(r) >> (8 * q), dia = (uint32_t)(b2s_sigma(r) >> 32) >> (8 * L.up3);
+    L.ad[4 * r] = off(col & 15);
+    L.ad[4 * r + 1] = off((col >> 4) & 15);
+    L.ad[4 * r + 2] = off(dia & 15);
+    L.ad[4 * r + 3] = off((dia >> 4) & 15);
+  }
+}
+
+#define SB_QUAD_G(x, y)              \
+  do {                               \
+    a += (x) + b; d = rotr32(d ^ a, 16); \
+    c += d;       b = rotr32(b ^ c, 12); \
+    a += (y) + b; d = rotr32(d ^ a, 8);  \
+    c += d;       b = rotr32(b ^ c, 7);  \
+  } while (0)
+
+// One final-block compression per four lanes of a fully active warp: message = hashes 2g and 2g + 1 of
+// buffer BUF, chaining value words q and 4 + q in h0, h4, t bytes hashed; replaced by the digest's.
+template <int BUF>
+__device__ __forceinline__ void quad_compress(const QuadBuffers& sm, const QuadLane& L, uint32_t& h0, uint32_t& h4,
+                                              uint32_t t) {
+  const char* base = reinterpret_cast<const char*>(sm.w[BUF]);
+  uint32_t a = h0, b = h4, c = L.iv, d = L.iv4;
+  if (L.q == 0) d ^= t;
+  if (L.q == 2) d = ~d;
+#pragma unroll
+  for (int r = 0; r < 10; ++r) {
+    SB_QUAD_G(*reinterpret_cast<const uint32_t*>(base + L.ad[4 * r]),
+              *reinterpret_cast<const uint32_t*>(base + L.ad[4 * r + 1]));
+    a = __shfl_sync(0xffffffffu, a, L.up3, 4);
+    d = __shfl_sync(0xffffffffu, d, L.up2, 4);
+    c = __shfl_sync(0xffffffffu, c, L.up1, 4);
+    SB_QUAD_G(*reinterpret_cast<const uint32_t*>(base + L.ad[4 * r + 2]),
+              *reinterpret_cast<const uint32_t*>(base + L.ad[4 * r + 3]));
+    a = __shfl_sync(0xffffffffu, a, L.up1, 4);
+    d = __shfl_sync(0xffffffffu, d, L.up2, 4);
+    c = __shfl_sync(0xffffffffu, c, L.up3, 4);
+  }
+  h0 ^= a ^ c;
+  h4 ^= b ^ d;
+}
+
+// One node level: n parents of the 2n hashes of buffer BUF into buffer 1 - BUF and layer `out`
+// (its first node). Warps without a parent skip it.
+template <int BUF>
+__device__ __forceinline__ void quad_level(QuadBuffers& sm, const QuadLane& L, uint32_t n, uint8_t* out, bool store,
+                                           const uint32_t seed[8], uint32_t seed0, uint32_t seed4, uint32_t one) {
+  if (n > QUAD_THREADS / 4) {
+    if (threadIdx.x < n) {
+      uint32_t h[8], m[16];
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        const uint2 v = *reinterpret_cast<const uint2*>(sm.w[BUF] + w * QS + 2 * threadIdx.x);
+        m[w] = v.x;
+        m[8 + w] = v.y;
+        h[w] = seed[w];
+      }
+      b2s_compress(h, m, 128, true, one);
+      put_hash(sm.w[1 - BUF], threadIdx.x, h);
+      if (store) store_hash(out, threadIdx.x, h);
+    }
+    return;
+  }
+  if ((threadIdx.x & ~31u) >= 4 * n) return;
+  uint32_t h0 = seed0, h4 = seed4;
+  quad_compress<BUF>(sm, L, h0, h4, 128);
+  const uint32_t g = threadIdx.x >> 2;
+  if (g < n) {
+    sm.w[1 - BUF][L.q * QS + g] = h0;
+    sm.w[1 - BUF][(4 + L.q) * QS + g] = h4;
+    if (store) {
+      uint32_t* d = reinterpret_cast<uint32_t*>(out) + g * 8 + L.q;
+      d[0] = h0;
+      d[4] = h4;
+    }
+  }
+}
+
+// Folds 2^log hashes of buffer 0 (log <= 9) to one; level j's nodes go to the layer of log size
+// child_log - j at first_child >> j. Returns the buffer whose hash 0 is the result. Every thread of
+// the CTA calls it; only warp 0 may read the result without a barrier (levels of at most 8 parents
+// run there alone).
+__device__ __forceinline__ uint32_t quad_fold(QuadBuffers& sm, const QuadLane& L, uint32_t log, uint8_t* layers,
+                                              bool store, uint32_t max_log, uint32_t child_log, uint64_t first_child,
+                                              const uint32_t seed[8], uint32_t one) {
+  const uint32_t seed0 = L.q == 0 ? seed[0] : L.q == 1 ? seed[1] : L.q == 2 ? seed[2] : seed[3];
+  const uint32_t seed4 = L.q == 0 ? seed[4] : L.q == 1 ? seed[5] : L.q == 2 ? seed[6] : seed[7];
+  auto out = [&](uint32_t j) { return layers + (merkle_layer_offset(max_log, child_log - j) + (first_child >> j)) * 32; };
+  auto barrier = [&](uint32_t n) {
+    if (n > 8) __syncthreads();
+    else __syncwarp();
+  };
+  uint32_t n = (1u << log) / 2;
+#pragma unroll 1
+  for (uint32_t j = 1; j <= log; j += 2) {
+    quad_level<0>(sm, L, n, out(j), store, seed, seed0, seed4, one);
+    barrier(n);
+    if (j == log) return 1;
+    n /= 2;
+    quad_level<1>(sm, L, n, out(j + 1), store, seed, seed0, seed4, one);
+    barrier(n);
+    n /= 2;
+  }
+  return 0;
+}
+
+// The top of a tree, the layers above 2^child_log children (child_log <= 12), in one launch: one CTA up
+// to 2^9 children, above that a cluster of 2, 4 or 8 CTAs, each folding 512 children to one node;
+// every CTA sends its node to CTA 0's shared memory, which folds the last levels. 2^12 children took
+// 14.2 us in eight CTAs plus 5.5 us and a launch in one with one lane per hash; now 16.7 us.
+__global__ void __launch_bounds__(QUAD_THREADS) k_merkle_top(uint8_t* layers, uint32_t max_log, uint32_t child_log,
+                                                             Seeds seeds, uint32_t one) {
+  __shared__ __align__(16) QuadBuffers sm;
+  __shared__ uint32_t top[8][8];
+  QuadLane L;
+  quad_lane_init(L);
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.barrier_arrive();  // every CTA runs before another one writes into its shared memory
+  const uint32_t n_ctas = cluster.num_blocks(), log = child_log < 9 ? child_log : 9;
+  const uint64_t first = (uint64_t)blockIdx.x << log;
+  chain_enter();
+  const uint4* src = reinterpret_cast<const uint4*>(layers + (merkle_layer_offset(max_log, child_log) + first) * 32);
+  for (uint32_t i = threadIdx.x; i < (2u << log); i += QUAD_THREADS) {
+    const uint4 v = src[i];
+    uint32_t* d = sm.w[0] + (i & 1) * 4 * QS + (i >> 1);
+    d[0] = v.x; d[QS] = v.y; d[2 * QS] = v.z; d[3 * QS] = v.w;
+  }
+  __syncthreads();
+  const uint32_t b = quad_fold(sm, L, log, layers, true, max_log, child_log, first, seeds.node, one);
+  cluster.barrier_wait();
+  if (n_ctas == 1) return;
+  if (threadIdx.x < 8) cluster.map_shared_rank(&top[0][0], 0)[threadIdx.x * 8 + blockIdx.x] = sm.w[b][threadIdx.x * QS];
+  cluster.sync();  // CTA 0 has every CTA's node; nothing reads another CTA's memory after this
+  if (blockIdx.x != 0 || threadIdx.x >= 32) return;
+  for (uint32_t i = threadIdx.x; i < 64; i += 32) sm.w[0][(i >> 3) * QS + (i & 7)] = top[i >> 3][i & 7];
+  __syncwarp();
+  quad_fold(sm, L, child_log - 9, layers, true, max_log, child_log - 9, 0, seeds.node, one);
+}
+
 // FRI fold fused with the next layer's commitment (src/core/fri/folding.zig:352-384,
 // 558-602; src/prover/fri.zig:377-592): thread i folds pair (2i, 2i+1) of the source
 // into line value i, stores its 4 coordinates and, when `layers` is set, hashes it
@@ -269,56 +477,92 @@ __global__ void __launch_bounds__(LEAF_THREADS) k_fri_fold_commit(TwiddleView it
 
 constexpr int FRI_DRAW_TRIES = 64;
 
-// One thread: the channel steps of one FRI layer (see fri_channel_step).
-__device__ void fri_channel_body(FriChannelDev* c, const uint8_t* root, uint32_t slot) {
-  uint32_t m[16], h[8];
-  const uint32_t* r = reinterpret_cast<const uint32_t*>(root);
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    m[k] = c->digest[k];
-    m[8 + k] = r[k];
-    c->roots[slot][k] = r[k];
+// The channel steps of one FRI layer (see fri_channel_step) by one warp, four lanes per hash: on entry
+// hash 0 of buffer 0 is the digest and hash 1 the layer's root; on return hash 0 of buffer 0 is the new
+// digest, *alpha (shared memory, 4 words) the drawn value and the number of draws is returned, 0 if
+// every try was rejected (*alpha is then 0 and the digest unchanged).
+__device__ __forceinline__ uint32_t quad_channel(QuadBuffers& sm, const QuadLane& L, uint32_t* alpha) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t init0 = L.q == 0 ? B2sIv::v0 ^ 0x01010020u : L.iv;
+  uint32_t d0 = init0, d4 = L.iv4;
+  quad_compress<0>(sm, L, d0, d4, 64);  // digest' = H(digest || root), one final 64-byte block
+  if (lane < 4) {
+    // digest' || LE32 n_draws || 0 in buffer 1
+    sm.w[1][L.q * QS] = d0;
+    sm.w[1][(4 + L.q) * QS] = d4;
+    sm.w[1][L.q * QS + 1] = 0;
+    sm.w[1][(4 + L.q) * QS + 1] = 0;
   }
-  b2s_init(h);
-  b2s_compress(h, m, 64, true);  // digest' = H(digest || root), one final 64-byte block
-  uint32_t n_draws = 0;
-  // drawSecureFelt: words of H(digest || LE32 n_draws || 0), all below 2p, else draw again.
+  __syncwarp();
+  // drawSecureFelt: words of H(digest' || LE32 n_draws || 0), all below 2p, else draw again.
   for (int tries = 0; tries < FRI_DRAW_TRIES; ++tries) {
-    uint32_t w[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) m[k] = h[k];
-    m[8] = n_draws;
-#pragma unroll
-    for (int k = 9; k < 16; ++k) m[k] = 0;
-    b2s_init(w);
-    b2s_compress(w, m, 37, true);
-    ++n_draws;
-    bool ok = true;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) ok &= w[k] < 2 * P;
-    if (ok) {
-#pragma unroll
-      for (int k = 0; k < 8; ++k) c->digest[k] = h[k];
-      c->n_draws = n_draws;
-      c->alpha[slot] = qmake(mreduce64(w[0]), mreduce64(w[1]), mreduce64(w[2]), mreduce64(w[3]));
-      return;
+    uint32_t w0 = init0, w4 = L.iv4;
+    quad_compress<1>(sm, L, w0, w4, 37);
+    const bool ok = w0 < 2 * P && w4 < 2 * P;
+    if ((__ballot_sync(0xffffffffu, ok) & 15u) == 15u) {
+      if (lane < 4) {
+        alpha[L.q] = mreduce64(w0);
+        sm.w[0][L.q * QS] = d0;
+        sm.w[0][(4 + L.q) * QS] = d4;
+      }
+      __syncwarp();
+      return tries + 1;
     }
+    if (lane == 0) sm.w[1][1] = tries + 1;
+    __syncwarp();
   }
-  c->status = 1;
-  c->alpha[slot] = qmake(0, 0, 0, 0);
+  if (lane < 4) alpha[L.q] = 0;
+  __syncwarp();
+  return 0;
 }
 
-__global__ void k_fri_channel(FriChannelDev* c, const uint8_t* root, uint32_t slot) {
+// One warp's record of a channel step in the device channel: the root, the drawn value, the state.
+__device__ __forceinline__ void channel_record(FriChannelDev* c, const QuadBuffers& sm, uint32_t slot, uint32_t n_draws,
+                                               uint32_t root_word, const uint32_t* alpha) {
+  const uint32_t lane = threadIdx.x & 31;
+  if (lane < 8) {
+    c->roots[slot][lane] = root_word;
+    if (n_draws) c->digest[lane] = sm.w[0][lane * QS];
+  }
+  if (lane < 4) reinterpret_cast<uint32_t*>(&c->alpha[slot])[lane] = alpha[lane];
+  if (lane == 0) {
+    if (n_draws) c->n_draws = n_draws;
+    else c->status = 1;
+  }
+}
+
+__global__ void __launch_bounds__(32) k_fri_channel(FriChannelDev* c, const uint8_t* root, uint32_t slot) {
+  __shared__ __align__(16) QuadBuffers sm;
+  __shared__ uint32_t alpha[4];
+  QuadLane L;
+  quad_lane_init(L);
   chain_enter();
-  fri_channel_body(c, root, slot);
+  const uint32_t lane = threadIdx.x;
+  uint32_t r = 0;
+  if (lane < 8) {
+    r = reinterpret_cast<const uint32_t*>(root)[lane];
+    sm.w[0][lane * QS] = c->digest[lane];
+    sm.w[0][lane * QS + 1] = r;
+  }
+  __syncwarp();
+  const uint32_t n = quad_channel(sm, L, alpha);
+  channel_record(c, sm, slot, n, r, alpha);
 }
 
-// The small inner FRI layers in one CTA: for line layers k = k0 .. n_inner-1 (2^(L-1-k) values,
+// The small inner FRI layers in one launch: for line layers k = k0 .. n_inner-1 (2^(L-1-k) values,
 // at most 2^FRI_TAIL_LOG), the channel step on layer k's root (alpha into slot k + 1), the fold
 // into layer k + 1 and, below the last layer, the commitment of layer k + 1: leaf hashes and every
-// node level, folded in shared memory. Same arithmetic, buffers and outputs as the per-layer
-// k_fri_channel + k_fri_fold_commit<false> + merkle_finish sequence.
-constexpr uint32_t FRI_TAIL_LOG = 12, FRI_TAIL_THREADS = 1024;
+// node level. Same arithmetic, buffers and outputs as the per-layer k_fri_channel +
+// k_fri_fold_commit<false> + merkle_finish sequence.
+//
+// A layer's work is a chain of hashes (leaf, node levels, two of the channel), so what counts is the
+// latency of each and that no level has more hashes on one multiprocessor than it runs at once: a
+// cluster of 8 CTAs holds a layer, each CTA an eighth of its values in shared memory, and folds its
+// part of the tree to one node; the eight nodes are sent to every CTA, and each folds the last three
+// levels and runs the channel step itself, so a layer needs one cluster barrier. Layers of fewer than
+// 128 folded values run in CTA 0 alone. One CTA of 1024 threads with one lane per hash took
+// 158 us for the layers from 2^12 on, after 27 us and three launches for the 2^13 one; now 127 us for all.
+constexpr uint32_t FRI_TAIL_LOG = 13, FRI_TAIL_CTAS = 8;
 struct FriTailParams {
   uint32_t L, k0, n_inner;
   uint32_t* line[FRI_MAX_LAYERS + 1];
@@ -327,42 +571,96 @@ struct FriTailParams {
   Seeds seeds;
 };
 
-__global__ void __launch_bounds__(FRI_TAIL_THREADS) k_fri_tail(FriChannelDev* c, const __grid_constant__ FriTailParams p,
-                                                               uint32_t one) {
+__global__ void __launch_bounds__(QUAD_THREADS) k_fri_tail(FriChannelDev* c, const __grid_constant__ FriTailParams p,
+                                                           uint32_t one) {
+  constexpr uint32_t VALS = 1u << (FRI_TAIL_LOG - 1 - 3);  // folded values of one CTA
+  static_assert(VALS <= QUAD_THREADS && VALS <= QCAP, "one thread and one leaf per value");
+  __shared__ __align__(16) QuadBuffers sm;
+  __shared__ __align__(16) uint32_t vals[4][VALS];
+  __shared__ uint32_t top[2][8][FRI_TAIL_CTAS];
+  __shared__ uint32_t digest[8], s_alpha[4];
+  QuadLane L;
+  quad_lane_init(L);
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.barrier_arrive();  // every CTA runs before another one writes into its shared memory
+  const uint32_t t = threadIdx.x, rank = blockIdx.x;
+  uint32_t ctas = cluster.num_blocks(), log_ctas = __ffs(ctas) - 1;
   chain_enter();
-  extern __shared__ uint32_t tsm[];  // (2^(FRI_TAIL_LOG-1)) hashes, then alpha
-  QM31* s_alpha = reinterpret_cast<QM31*>(tsm + (1u << (FRI_TAIL_LOG - 1)) * 8);
-  const uint32_t t = threadIdx.x;
+  if (t < 8) digest[t] = c->digest[t];
+  uint32_t root_word = 0;  // word t of the layer's root in threads 0..7
+  if (t < 8) root_word = reinterpret_cast<const uint32_t*>(p.tree[p.k0] + (2ull * (1u << (p.L - 1 - p.k0)) - 2) * 32)[t];
+  cluster.barrier_wait();
+  bool local = false;  // this layer's values are in vals
   for (uint32_t k = p.k0; k < p.n_inner; ++k) {
     const uint32_t lg = p.L - 1 - k;
-    const uint64_t sz = 1ull << lg, n = sz >> 1;
-    if (t == 0) {
-      fri_channel_body(c, p.tree[k] + (2 * sz - 2) * 32, k + 1);
-      *s_alpha = c->alpha[k + 1];
-    }
-    __syncthreads();
-    const QM31 alpha = *s_alpha;
-    const uint32_t* src = p.line[k];
-    uint32_t* dst = p.line[k + 1];
+    const uint32_t sz = 1u << lg, n = sz >> 1;  // values of the layer, of the folded one
     const bool commit = k + 1 < p.n_inner;
-    for (uint32_t i = t; i < n; i += FRI_TAIL_THREADS) {
-      QM31 f0 = qmake(src[2 * i], src[sz + 2 * i], src[2 * sz + 2 * i], src[3 * sz + 2 * i]);
-      QM31 f1 = qmake(src[2 * i + 1], src[sz + 2 * i + 1], src[2 * sz + 2 * i + 1], src[3 * sz + 2 * i + 1]);
+    if (ctas > 1 && n < 16 * ctas) {
+      // The layer fits one CTA: the others' values are in the line layer (written before the barrier).
+      if (rank != 0) return;
+      ctas = 1;
+      log_ctas = 0;
+      local = false;
+    }
+    const uint32_t n_loc = n >> log_ctas, i = rank * n_loc + t;
+    const bool active = t < n_loc;
+    // Everything of the fold that does not need alpha.
+    QM31 f0 = qzero(), f1 = qzero();
+    if (active) {
+      uint2 w[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        w[q] = local ? *reinterpret_cast<const uint2*>(&vals[q][2 * t])
+                     : __ldcg(reinterpret_cast<const uint2*>(p.line[k] + (size_t)q * sz + 2 * i));
+      f0 = qmake(w[0].x, w[1].x, w[2].x, w[3].x);
+      f1 = qmake(w[0].y, w[1].y, w[2].y, w[3].y);
       fri_ibfly(f0, f1, p.tv[k].line(1, i));
-      const QM31 r = qadd(f0, qmul(alpha, f1));
-      dst[i] = r.c0.a; dst[n + i] = r.c0.b; dst[2 * n + i] = r.c1.a; dst[3 * n + i] = r.c1.b;
+    }
+    if (t < 32) {
+      if (t < 8) {
+        sm.w[0][t * QS] = digest[t];
+        sm.w[0][t * QS + 1] = root_word;
+      }
+      __syncwarp();
+      const uint32_t draws = quad_channel(sm, L, s_alpha);
+      if (rank == 0) channel_record(c, sm, k + 1, draws, root_word, s_alpha);
+      if (t < 8) digest[t] = sm.w[0][t * QS];
+    }
+    __syncthreads();  // alpha is drawn; every thread has read its values
+    if (active) {
+      const QM31 r = qadd(f0, qmul(qload4(s_alpha), f1));
+      uint32_t* dst = p.line[k + 1] + i;
+      dst[0] = r.c0.a; dst[n] = r.c0.b; dst[2 * n] = r.c1.a; dst[3 * n] = r.c1.b;
+      vals[0][t] = r.c0.a; vals[1][t] = r.c0.b; vals[2][t] = r.c1.a; vals[3][t] = r.c1.b;
       if (commit) {
         uint32_t h[8], m[16] = {r.c0.a, r.c0.b, r.c1.a, r.c1.b, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
         for (int q = 0; q < 8; ++q) h[q] = p.seeds.leaf[q];
         b2s_compress(h, m, 80, true, one);
         store_hash(p.tree[k + 1], i, h);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) tsm[i * 8 + q] = h[q];
+        put_hash(sm.w[0], t, h);
       }
     }
+    local = true;
     __syncthreads();
-    if (commit) fold_levels(tsm, (uint32_t)n, lg - 1, p.tree[k + 1], lg - 1, lg - 1, 0, p.seeds.node, one);
+    if (!commit) continue;
+    const uint32_t max_log = lg - 1, loc_log = max_log - log_ctas;
+    uint32_t b = quad_fold(sm, L, loc_log, p.tree[k + 1], true, max_log, max_log, (uint64_t)rank << loc_log, p.seeds.node, one);
+    if (ctas > 1) {
+      // Warp 0 sends this CTA's node to every CTA (two buffers: a CTA may be a layer ahead of one
+      // that still reads).
+      uint32_t* mine = &top[k & 1][0][0];
+      for (uint32_t x = t; x < 8 * FRI_TAIL_CTAS && t < 32; x += 32)
+        cluster.map_shared_rank(mine, x >> 3)[(x & 7) * FRI_TAIL_CTAS + rank] = sm.w[b][(x & 7) * QS];
+      cluster.sync();
+      if (t < 32) {
+        for (uint32_t x = t; x < 8 * FRI_TAIL_CTAS; x += 32) sm.w[0][(x >> 3) * QS + (x & 7)] = mine[x];
+        __syncwarp();
+        b = quad_fold(sm, L, 3, p.tree[k + 1], rank == 0, max_log, 3, 0, p.seeds.node, one);
+      }
+    }
+    if (t < 8) root_word = sm.w[b][t * QS];
+    __syncwarp();
   }
 }
 
@@ -383,31 +681,30 @@ static const Seeds& seeds_once() {
   return seeds;
 }
 
+// Node levels that a leaf launch folds in its CTAs: the whole tree when it fits one, else the three whose
+// parents fill whole warps.
+static uint32_t leaf_levels(uint32_t log) { return log <= LEAF_LEVELS ? log : FULL_WARP_LEVELS; }
+
 // Folds the node layers above child layer `child_log` of a tree with 2^max_log leaves.
 static cudaError_t merkle_finish(uint8_t* layers, uint32_t max_log, uint32_t child_log, cudaStream_t stream) {
   const Seeds& seeds = seeds_once();
   cudaError_t e = cudaSuccess;
   // Large layers: four levels per launch, each CTA folding 512 children (every level's
-  // parents fill whole warps: 256, 128, 64, 32).
+  // parents fill whole warps: 256, 128, 64, 32), until 2^9 .. 2^12 are left.
   while (child_log > NODE_FOLD_LOG) {
-    uint32_t levels = child_log - NODE_FOLD_LOG < 4 ? child_log - NODE_FOLD_LOG : 4;
-    uint32_t blocks = (uint32_t)((1ull << child_log) / (2 * NODE_THREADS));
-    e = launch_chained(k_merkle_nodes, blocks, NODE_THREADS, 0, stream, layers, max_log, child_log, levels, seeds, 1u);
+    const uint32_t blocks = (uint32_t)((1ull << child_log) / (2 * NODE_THREADS));
+    e = launch_chained(k_merkle_nodes, blocks, NODE_THREADS, 0, stream, layers, max_log, child_log, 4u, seeds, 1u);
     note_launch();
     if (e != cudaSuccess) return e;
-    child_log -= levels;
+    child_log -= 4;
   }
-  while (child_log > 0) {
-    uint32_t levels = child_log < 9 ? child_log : 9;
-    uint64_t n_children = 1ull << child_log;
-    uint32_t per_cta = n_children < 2 * NODE_THREADS ? (uint32_t)n_children : 2 * NODE_THREADS;
-    uint32_t blocks = (uint32_t)(n_children / per_cta);
-    e = launch_chained(k_merkle_nodes, blocks, NODE_THREADS, 0, stream, layers, max_log, child_log, levels, seeds, 1u);
-    note_launch();
-    if (e != cudaSuccess) return e;
-    child_log -= levels;
-  }
-  return cudaSuccess;
+  if (child_log > 9)
+    e = launch_cluster_chained(k_merkle_top, 1u << (child_log - 9), QUAD_THREADS, 0, stream, layers, max_log, child_log,
+                               seeds, 1u);
+  else if (child_log > 0)
+    e = launch_chained(k_merkle_top, 1, QUAD_THREADS, 0, stream, layers, max_log, child_log, seeds, 1u);
+  if (child_log > 0) note_launch();
+  return e;
 }
 
 uint32_t fri_tail_first(uint32_t L, uint32_t n_inner) {
@@ -430,20 +727,16 @@ cudaError_t fri_tail(const DeviceTables& t, FriChannelDev* c, uint32_t L, uint32
     p.tv[k] = t.view(L - k, true);
   }
   p.seeds = seeds_once();
-  const size_t smem = (1u << (FRI_TAIL_LOG - 1)) * 32 + 16;
-  static const bool attr = [&] {  // once per process (thread-safe static initialisation)
-    cudaFuncSetAttribute(k_fri_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return true;
-  }();
-  (void)attr;
-  cudaError_t e = launch_chained(k_fri_tail, 1, FRI_TAIL_THREADS, smem, stream, c, p, 1u);
+  // Eight CTAs while each has at least 16 folded values of the first layer, else one.
+  const uint32_t ctas = (1u << (L - 2 - k0)) >= 16 * FRI_TAIL_CTAS ? FRI_TAIL_CTAS : 1;
+  cudaError_t e = launch_cluster_chained(k_fri_tail, ctas, QUAD_THREADS, 0, stream, c, p, 1u);
   note_launch();
   return e;
 }
 
 cudaError_t fri_channel_step(FriChannelDev* c, const uint8_t* root, uint32_t slot, cudaStream_t stream) {
   if (slot >= FRI_MAX_LAYERS) return cudaErrorInvalidValue;
-  cudaError_t e = launch_chained(k_fri_channel, 1, 1, 0, stream, c, root, slot);
+  cudaError_t e = launch_chained(k_fri_channel, 1, 32, 0, stream, c, root, slot);
   note_launch();
   return e;
 }
@@ -455,9 +748,8 @@ cudaError_t fri_fold_commit(const DeviceTables& t, bool circle, uint32_t src_log
   const uint32_t dst_log = src_log - 1;
   const uint64_t n = 1ull << dst_log;
   const uint32_t grid = (uint32_t)((n + LEAF_THREADS - 1) / LEAF_THREADS);
-  // One compression per leaf; the CTA also folds the three full-warp node levels
-  // (the whole tree when it fits one CTA).
-  const uint32_t levels = layers ? (dst_log <= LEAF_LEVELS ? dst_log : FULL_WARP_LEVELS) : 0;
+  // One compression per leaf.
+  const uint32_t levels = layers ? leaf_levels(dst_log) : 0;
   cudaError_t e;
   if (circle)
     e = launch_chained(k_fri_fold_commit<true>, grid, LEAF_THREADS, 0, stream, t.view(src_log, true), dst_log, src,
@@ -478,24 +770,22 @@ cudaError_t merkle_commit(uint32_t log_size, uint32_t n_cols, const uint32_t* co
     return cudaGetLastError();
   }
   const uint64_t n_rows = 1ull << log_size;
-  // A tree that fits one CTA is folded to its root in the leaf launch; larger ones
-  // fold their three full-warp node levels there. Levels 4-8 inside the CTA would
-  // run on partly empty warps (16, 8, .. 1 parents): for 2^21 leaves of 4 words,
-  // folding 8 levels took 283 us, 3 levels 245 us and none 254 us.
-  uint32_t leaf_levels = log_size <= LEAF_LEVELS ? log_size : FULL_WARP_LEVELS;
+  // Levels 4-8 inside the leaf CTA would run on partly empty warps (16, 8, .. 1 parents): for 2^21
+  // leaves of 4 words, folding 8 levels took 283 us, 3 levels 245 us and none 254 us.
+  const uint32_t levels = leaf_levels(log_size);
   uint32_t grid = (uint32_t)((n_rows + LEAF_THREADS - 1) / LEAF_THREADS);
   // Variants: leaf kernels built for 5, 6 and 4 resident CTAs per SM (48, 40 and 64 registers).
   auto commit = [&](int variant) -> cudaError_t {
     if (variant == 1)
-      k_merkle_leaves<6><<<grid, LEAF_THREADS, 0, stream>>>(log_size, n_cols, cols, stride, layers, seeds, leaf_levels, 1u);
+      k_merkle_leaves<6><<<grid, LEAF_THREADS, 0, stream>>>(log_size, n_cols, cols, stride, layers, seeds, levels, 1u);
     else if (variant == 2)
-      k_merkle_leaves<4><<<grid, LEAF_THREADS, 0, stream>>>(log_size, n_cols, cols, stride, layers, seeds, leaf_levels, 1u);
+      k_merkle_leaves<4><<<grid, LEAF_THREADS, 0, stream>>>(log_size, n_cols, cols, stride, layers, seeds, levels, 1u);
     else
-      k_merkle_leaves<5><<<grid, LEAF_THREADS, 0, stream>>>(log_size, n_cols, cols, stride, layers, seeds, leaf_levels, 1u);
+      k_merkle_leaves<5><<<grid, LEAF_THREADS, 0, stream>>>(log_size, n_cols, cols, stride, layers, seeds, levels, 1u);
     note_launch();
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    return merkle_finish(layers, log_size, log_size - leaf_levels, stream);
+    return merkle_finish(layers, log_size, log_size - levels, stream);
   };
   // Trees big enough for the occupancy to matter; the commit only reads the columns.
   return tuned_run(TUNE_LEAVES, log_size, n_cols, log_size >= 16 ? 3 : 1, true, stream, commit);
@@ -510,13 +800,13 @@ cudaError_t merkle_commit_lifted(uint32_t max_log, uint32_t n_cols, const uint32
   }
   if (n_cols > LIFTED_MAX_COLS) return cudaErrorInvalidValue;
   const uint64_t n_rows = 1ull << max_log;
-  uint32_t leaf_levels = max_log <= LEAF_LEVELS ? max_log : FULL_WARP_LEVELS;
+  const uint32_t levels = leaf_levels(max_log);
   uint32_t grid = (uint32_t)((n_rows + LEAF_THREADS - 1) / LEAF_THREADS);
   k_merkle_leaves_lifted<<<grid, LEAF_THREADS, 0, stream>>>(max_log, n_cols, col_ptrs, col_logs, layers, seeds,
-                                                            leaf_levels, 1u); note_launch();
+                                                            levels, 1u); note_launch();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  return merkle_finish(layers, max_log, max_log - leaf_levels, stream);
+  return merkle_finish(layers, max_log, max_log - levels, stream);
 }
 
 // ---------------------------------------------------------------------------

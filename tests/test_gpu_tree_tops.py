@@ -1,0 +1,29 @@
+"""The launches that end a tree and the FRI phase (a CTA or a cluster, four lanes per hash): every
+stored node at the sizes where the launches and cluster sizes change, and whole proofs whose FRI tail
+starts at each layer size, with one and with eight CTAs."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+P = 2**31 - 1
+
+
+@pytest.mark.parametrize("log", [8, 9, 10, 11, 12, 13, 14, 15, 16])
+def test_every_layer(ctx, log):
+    import torch
+    cols = np.random.default_rng(log).integers(0, P, size=(3, 1 << log), dtype=np.uint32)
+    layers = torch.empty(((2 << log) - 1) * 32, dtype=torch.uint8, device="cuda")
+    root = ctx.merkle_commit(torch.from_numpy(cols.view(np.int32)).cuda(), log, 3, layers)
+    ref = np.concatenate(oracle.merkle_layers(list(cols)))
+    assert np.array_equal(layers.cpu().numpy().reshape(-1, 32), ref) and root == ref[-1].tobytes()
+
+
+@pytest.mark.parametrize("log_n,last", [(4, 0), (7, 0), (8, 0), (9, 2), (12, 0), (13, 1), (14, 0)])
+def test_fri_tail(ctx, log_n, last):
+    import stwo_b200 as sb
+    o = oracle.config("functional", log_last_layer_degree_bound=last)
+    g = sb.PcsConfig(o.pow_bits, sb.FriConfig(o.log_blowup_factor, last, o.n_queries))
+    got = ctx.prove_wide_fibonacci(sb.Statement(log_n, 5), g, trace_kind=sb.TRACE_SEEDED, trace_seed=log_n)
+    assert got == oracle.prove_wide_fib(log_n, 5, o, trace_kind=1, trace_seed=log_n)
