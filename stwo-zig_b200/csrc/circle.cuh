@@ -25,12 +25,9 @@ SB_HD uint32_t subgroup_gen(uint32_t log_size) { return 1u << (CIRCLE_LOG_ORDER 
 // Device/host view of the point table: table[0 .. LO) = lo * G, table[LO .. LO + HI) = (hi 2^16) G.
 struct PointTable {
   const PointM* t;
-  SB_HD PointM at(uint32_t idx) const {
-    idx &= INDEX_MASK;
-    PointM lo = t[idx & (POINT_TABLE_LO - 1)];
-    PointM hi = t[POINT_TABLE_LO + (idx >> POINT_TABLE_LO_BITS)];
-    return padd(lo, hi);
-  }
+  SB_HD PointM lo(uint32_t idx) const { return t[idx & (POINT_TABLE_LO - 1)]; }
+  SB_HD PointM hi(uint32_t idx) const { return t[POINT_TABLE_LO + ((idx & INDEX_MASK) >> POINT_TABLE_LO_BITS)]; }
+  SB_HD PointM at(uint32_t idx) const { return padd(lo(idx), hi(idx)); }
 };
 
 inline std::vector<PointM> build_point_table() {

@@ -106,7 +106,7 @@ struct QuotientBatchDev {
 // Single-size quotient: all columns have log size `log_size` (the lifting size).
 // col_ptrs/coeff_c are device arrays of length n_entries; batches device array.
 // `status` (device word, may be null): a caller that passes one vouches that every column pointer is
-// 16-byte aligned, which makes the bulk-staged kernel one of the tuned variants; that kernel ORs
+// 16-byte aligned, which allows 16-byte copies of them and, as a forced variant, the bulk-staged kernel, which ORs
 // QUOT_STATUS_* bits into it when a staged load runs out of time or the batches do not fit its
 // item table, and its output is then not valid.
 constexpr uint32_t QUOT_STATUS_TIMEOUT = 2, QUOT_STATUS_LAYOUT = 4;

@@ -9,6 +9,7 @@
 
 #include "blake2s.cuh"
 #include "kernels.cuh"
+#include "mma_dot.cuh"
 #include "tuner.hpp"
 
 namespace sb {
@@ -117,96 +118,156 @@ __global__ void __launch_bounds__(256) k_composition(uint32_t log_n, uint32_t W,
   }
 }
 
-// R consecutive rows per thread (RowVec<R>; R = 2 with 8-byte loads measured best:
-// more warps and more loads in flight than 4 rows with 16-byte loads), the column
-// loop unrolled by U (a multiple of 3: U loads in flight before their use, a
-// 64-bit fold per three terms) and each column's square computed once (it is b^2
-// of one constraint and a^2 of the next). Needs columns and output aligned to R
-// words (eval, stride, out, out_stride) and 2^(log_n+1) >= R.
-template <int R>
-struct RowVec;
-template <>
-struct RowVec<2> {
-  uint2 v;
-  __device__ __forceinline__ static RowVec load(const uint32_t* p) { return {__ldg(reinterpret_cast<const uint2*>(p))}; }
-  __device__ __forceinline__ static RowVec load_words(const uint32_t* p) { return {make_uint2(__ldg(p), __ldg(p + 1))}; }
-  __device__ __forceinline__ uint32_t operator[](int j) const { return j == 0 ? v.x : v.y; }
-  __device__ __forceinline__ static void store(uint32_t* p, const uint32_t* w) {
-    *reinterpret_cast<uint2*>(p) = make_uint2(w[0], w[1]);
+// The same sums on the tensor cores (mma_dot.cuh). A constraint is linear in the columns and their
+// squares, so sum_k coeff_k (c_{k+2} - c_k^2 - c_{k+1}^2) = sum_c (alpha_c v_c + beta_c v_c^2) with
+// alpha_c = coeff_{c-2} and beta_c = -(coeff_c + coeff_{c-1}) (a coefficient outside 0 .. W-3 is zero):
+// two products per column with coefficients that are the same for every row. The square enters as any
+// 32-bit word congruent to it, so it is folded once and not made canonical.
+//
+// Bound by HBM and the integer mma rate: 2^21 rows x 100 columns 207 us, 4.2 TB/s (the kernel with
+// lazily accumulated 64-bit multiply-adds, two rows per thread, 243 us).
+constexpr int MMA_THREADS = 128;
+
+// The words of a step (64 rows of eight columns), STAGES steps ahead: each warp copies them
+// asynchronously into a ring of its own in shared memory, so that it keeps 2 KB a stage in flight across steps
+// and row blocks without block barriers and without registers for them. The copies' lanes follow memory
+// (sixteen lanes a column, 256 bytes; two columns per instruction) and the operand lanes read back
+// theirs; columns lie 288 bytes apart, which puts the sixteen lanes of a read phase on distinct banks.
+// A read-only probe of this walk (108 columns of 2^21 rows) runs at 6.9 TB/s; with each lane copying its
+// own operand words (neighbour lanes on four different columns) it stays at 3.9 TB/s at any depth, and
+// with the same depth in registers the quotients took 325 us.
+// Stages of the composition (four CTAs per SM: 124 registers) and of the quotients (three: 168).
+constexpr int COMP_STAGES = 4, QUOT_STAGES = 6;
+constexpr uint32_t MMA_ROWS = 64;           // rows of a warp's block
+constexpr uint32_t MMA_COL = 4 * MMA_ROWS + 32;   // bytes between a stage's columns
+constexpr uint32_t MMA_STAGE = 8 * MMA_COL;       // bytes of a warp's stage
+constexpr uint32_t mma_ring_bytes(int stages) { return (MMA_THREADS / 32) * stages * MMA_STAGE; }
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+template <int STAGES>
+class WordRing {
+ public:
+  __device__ __forceinline__ explicit WordRing(const void* ring) : in_(0), out_(0) {
+    const uint32_t lane = threadIdx.x & 31;
+    const char* warp = static_cast<const char*>(ring) + (threadIdx.x >> 5) * (STAGES * MMA_STAGE);
+    put_ = smem_u32(warp) + (lane >> 4) * MMA_COL + (lane & 15) * 16;
+    get_ = warp + (lane & 3) * MMA_COL + (lane >> 2) * 8;
   }
+  // Column of a step (before the pair's number) and row of the block that this lane copies.
+  __device__ __forceinline__ static uint32_t column() { return (threadIdx.x & 31) >> 4; }
+  __device__ __forceinline__ static uint32_t row() { return 4 * (threadIdx.x & 15); }
+  // Starts the copy of this lane's four rows of column 2 u + column() of the step (16-byte aligned when ALIGNED).
+  template <bool ALIGNED>
+  __device__ __forceinline__ void fetch(int u, const uint32_t* src) {
+    const uint32_t d = put_ + in_ + u * 2 * MMA_COL;
+    if (ALIGNED) {
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + 4 * k), "l"(src + k) : "memory");
+    }
+  }
+  // Ends a step's copies (also of none): one per step, in order.
+  __device__ __forceinline__ void commit() {
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    in_ = in_ + MMA_STAGE == STAGES * MMA_STAGE ? 0 : in_ + MMA_STAGE;
+  }
+  // This lane's words of the oldest step not yet taken; its slots are then free for the next fetch.
+  __device__ __forceinline__ void take(mmadot::Words& w) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
+    __syncwarp();  // every lane's copies of the step have landed
+    const char* s = get_ + out_;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const uint2 lo = *reinterpret_cast<const uint2*>(s + 64 * m), hi = *reinterpret_cast<const uint2*>(s + 4 * MMA_COL + 64 * m);
+      w.a[m] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+    }
+    out_ = out_ + MMA_STAGE == STAGES * MMA_STAGE ? 0 : out_ + MMA_STAGE;
+    __syncwarp();  // every lane has read its words
+  }
+
+ private:
+  uint32_t put_, in_, out_;
+  const char* get_;
 };
 
-// Rows per thread and unroll depth of the vectorized composition and quotient kernels.
-constexpr int COMP_R = 2, COMP_U = 6, QUOT_R = 2, QUOT_U = 6;
+template <bool ALIGNED>
+__device__ __forceinline__ void store_rows2(uint32_t* p, uint2 v) {
+  if (ALIGNED) { *reinterpret_cast<uint2*>(p) = v; return; }
+  p[0] = v.x; p[1] = v.y;
+}
 
-template <int R, int U>
-__global__ void __launch_bounds__(256, 4) k_composition_v(uint32_t log_n, uint32_t W, const uint32_t* __restrict__ eval,
-                                                          uint64_t stride, const QM31* __restrict__ coeffs,
-                                                          uint32_t den0, uint32_t den1, uint32_t* out,
-                                                          uint64_t out_stride) {
-  static_assert(U % 3 == 0, "fold every three terms");
-  using V = RowVec<R>;
-  extern __shared__ uint4 scq[];  // W-2 coefficients
-  const uint32_t n_cons = W - 2;
-  for (uint32_t i = threadIdx.x; i < n_cons; i += blockDim.x) {
-    QM31 c = coeffs[i];
-    scq[i] = make_uint4(c.c0.a, c.c0.b, c.c1.a, c.c1.b);
+// A word below 2^32 congruent to a^2 (a < p): 2 a^2 = hi 2^32 + lo gives a^2 = hi + lo / 2 (mod p).
+__device__ __forceinline__ uint32_t square_word(uint32_t a) {
+  const uint64_t x = (uint64_t)a * (a + a);
+  return (uint32_t)(x >> 32) + ((uint32_t)x >> 1);
+}
+__device__ __forceinline__ uint4 square_word4(uint4 v) {
+  return make_uint4(square_word(v.x), square_word(v.y), square_word(v.z), square_word(v.w));
+}
+
+// Byte-reversed coordinate words of a coefficient.
+__device__ __forceinline__ void put_reversed(uint32_t* d, QM31 c) {
+  d[0] = mmadot::byte_reverse(c.c0.a); d[1] = mmadot::byte_reverse(c.c0.b);
+  d[2] = mmadot::byte_reverse(c.c1.a); d[3] = mmadot::byte_reverse(c.c1.b);
+}
+
+// Needs 2^(log_n+1) >= 64 rows; ALIGNED: columns and output 16-byte aligned with strides of a multiple
+// of four words.
+template <bool ALIGNED>
+__global__ void __launch_bounds__(MMA_THREADS, 4) k_composition_mma(uint32_t log_n, uint32_t W,
+                                                                    const uint32_t* __restrict__ eval, uint64_t stride,
+                                                                    const QM31* __restrict__ coeffs, uint32_t den0,
+                                                                    uint32_t den1, uint32_t* out, uint64_t out_stride) {
+  extern __shared__ uint4 scm[];  // the ring, then alpha, then beta, of the columns padded to a multiple of 8
+  const uint32_t steps = (W + 7) / 8, n_cons = W - 2;
+  uint32_t* alpha = reinterpret_cast<uint32_t*>(scm + mma_ring_bytes(COMP_STAGES) / 16);
+  uint32_t* beta = alpha + 32 * steps;
+  for (uint32_t c = threadIdx.x; c < 8 * steps; c += MMA_THREADS) {
+    auto coeff = [&](uint32_t k) { return k < n_cons ? coeffs[k] : qzero(); };  // k wraps above for c < 2
+    put_reversed(alpha + 4 * c, c < W ? coeff(c - 2) : qzero());
+    put_reversed(beta + 4 * c, c < W ? qneg(qadd(coeff(c), coeff(c - 1))) : qzero());
   }
   __syncthreads();
-  const uint32_t groups = (2u << log_n) / R;
-  for (uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x; gi < groups; gi += gridDim.x * blockDim.x) {
-    const uint32_t row0 = gi * R;
-    const uint32_t* base = eval + row0;
-    V A = V::load(base), B = V::load(base + stride);
-    uint32_t sa[R], sb[R];
+  const uint32_t lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const mmadot::LaneShifts shifts = mmadot::lane_shifts(g & 1);
+  const uint32_t n_blocks = (2u << log_n) / MMA_ROWS, warps = gridDim.x * (MMA_THREADS / 32);
+  const uint32_t first_blk = blockIdx.x * (MMA_THREADS / 32) + (threadIdx.x >> 5);
+  WordRing<COMP_STAGES> ring(scm);
+  uint32_t p_blk = first_blk, p_step = 0;  // next step to load
+  auto fetch = [&]() {
+    if (p_blk < n_blocks) {
+      // Padding columns (zero coefficients) read the last column.
+      const uint32_t* rows = eval + MMA_ROWS * p_blk + ring.row();
 #pragma unroll
-    for (int j = 0; j < R; ++j) { sa[j] = mmul(A[j], A[j]); sb[j] = mmul(B[j], B[j]); }
-    uint64_t acc[R][4];
-#pragma unroll
-    for (int j = 0; j < R; ++j)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[j][c] = 0;
-    auto step = [&](const V& C, const uint4& q) {
-#pragma unroll
-      for (int j = 0; j < R; ++j) {
-        uint32_t cj = C[j];
-        uint32_t cons = msub(cj, madd(sa[j], sb[j]));
-        sa[j] = sb[j];
-        sb[j] = mmul(cj, cj);
-        acc[j][0] += (uint64_t)q.x * cons;
-        acc[j][1] += (uint64_t)q.y * cons;
-        acc[j][2] += (uint64_t)q.z * cons;
-        acc[j][3] += (uint64_t)q.w * cons;
-      }
-    };
-    auto fold = [&]() {
-#pragma unroll
-      for (int j = 0; j < R; ++j)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[j][c] = mfold64(acc[j][c]);
-    };
-    uint32_t k = 0;
-    for (; k + U <= n_cons; k += U) {
-      V C[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) C[u] = V::load(base + (uint64_t)(k + 2 + u) * stride);
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        step(C[u], scq[k + u]);
-        if (u % 3 == 2) fold();
-      }
+      for (int u = 0; u < 4; ++u)
+        ring.fetch<ALIGNED>(u, rows + (uint64_t)min(8 * p_step + 2 * u + ring.column(), W - 1) * stride);
+      if (++p_step == steps) { p_step = 0; p_blk += warps; }
     }
-    for (uint32_t t = 0; k < n_cons; ++k, ++t) {
-      step(V::load(base + (uint64_t)(k + 2) * stride), scq[k]);
-      if (t % 3 == 2) fold();
+    ring.commit();
+  };
+  for (int d = 0; d < COMP_STAGES; ++d) fetch();
+  for (uint32_t blk = first_blk; blk < n_blocks; blk += warps) {
+    const uint32_t row0 = MMA_ROWS * blk + 2 * g;
+    mmadot::Acc acc;
+    acc.clear();
+    const uint32_t* qa = alpha + 4 * t + (g >> 1);
+    const uint32_t* qb = beta + 4 * t + (g >> 1);
+    for (uint32_t s = 0; s < steps; ++s, qa += 32, qb += 32) {
+      mmadot::Words w;
+      ring.take(w);
+      acc.step(w, qa[0], qa[16], shifts);
+      fetch();
+#pragma unroll
+      for (int m = 0; m < 4; ++m) w.a[m] = square_word4(w.a[m]);
+      acc.step(w, qb[0], qb[16], shifts);
     }
-    const uint32_t d = (row0 >> log_n) ? den1 : den0;  // the R rows share row >> log_n
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      uint32_t w[R];
-#pragma unroll
-      for (int j = 0; j < R; ++j) w[j] = mmul(mreduce64(acc[j][c]), d);
-      V::store(out + (uint64_t)c * out_stride + row0, w);
+    for (int m = 0; m < 4; ++m) {
+      const uint32_t row = row0 + 16 * m, den = (row >> log_n) ? den1 : den0;  // both rows share row >> log_n
+      store_rows2<ALIGNED>(out + t * out_stride + row,
+                           make_uint2(mmul(mmadot::row_sum(acc, m, 0), den), mmul(mmadot::row_sum(acc, m, 1), den)));
     }
   }
 }
@@ -414,101 +475,105 @@ __device__ __forceinline__ void quot_batch_finish(const QuotientBatchDev& bt, co
   }
 }
 
-// R consecutive rows per thread: 8- or 16-byte loads of every column, entries
-// unrolled by U (U loads in flight), and the R rows' denominators inverted
-// together (one CM31 inversion per R rows, Montgomery's trick; a zero product
-// falls back to per-row inversion so a zero denominator gives the same zero as
-// the one-row kernel). Needs an output aligned to R words and 2^log_size >= R; a
-// CTA that finds a column pointer off the vector alignment loads word by word.
-template <int R, int U, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_quotients_v(PointTable pts, uint32_t log_size, uint32_t n_batches,
-                                                        const QuotientBatchDev* __restrict__ batches,
-                                                        const uint32_t* const* __restrict__ col_ptrs,
-                                                        const QM31* __restrict__ coeff_c, uint32_t* out,
-                                                        uint64_t out_stride) {
-  static_assert(U % 3 == 0, "fold every three terms");
-  using V = RowVec<R>;
-  extern __shared__ uint4 sqe[];  // QUOT_MAX_ENTRIES coefficients, then the column pointers
-  const uint32_t** sptr = reinterpret_cast<const uint32_t**>(sqe + QUOT_MAX_ENTRIES);
-  __shared__ int s_bad;
-  uint32_t n_entries = 0;
-  for (uint32_t b = 0; b < n_batches; ++b) n_entries = max(n_entries, batches[b].first + batches[b].count);
-  if (threadIdx.x == 0) s_bad = 0;
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < n_entries; i += blockDim.x) {
-    QM31 c = coeff_c[i];
-    sqe[i] = make_uint4(c.c0.a, c.c0.b, c.c1.a, c.c1.b);
-    const uint32_t* p = col_ptrs[i];
-    sptr[i] = p;
-    if (reinterpret_cast<uintptr_t>(p) & (4 * R - 1)) s_bad = 1;
+// The quotients of 64 rows per warp, the numerators' sums on the tensor cores (mma_dot.cuh): lane (g, t)
+// ends with coordinate t of rows 16m + 2g and + 1 for m = 0..3. A batch's entries are taken eight columns a step, padded
+// with zero coefficients. Lane t inverts the denominators of tile t's two rows, whose points are
+// conjugates, with one inversion, and the four lanes exchange them. ALIGNED: columns and output 16-byte aligned, with strides of a multiple of four words.
+//
+// Bound by HBM: 2^21 rows x 108 columns 168 us, 5.6 TB/s (the lazily accumulating register
+// kernel, ten instructions per word, 265 us; the bulk-staged one 258 us).
+template <bool ALIGNED>
+__global__ void __launch_bounds__(MMA_THREADS, 3) k_quotients_mma(PointTable pts, uint32_t log_size, uint32_t n_batches,
+                                                                  const QuotientBatchDev* __restrict__ batches,
+                                                                  const uint32_t* const* __restrict__ col_ptrs,
+                                                                  const QM31* __restrict__ coeff_c, uint32_t padded,
+                                                                  uint32_t* out, uint64_t out_stride) {
+  extern __shared__ uint4 qmma[];
+  uint32_t* sq = reinterpret_cast<uint32_t*>(qmma + mma_ring_bytes(QUOT_STAGES) / 16);  // byte-reversed coefficients
+  const uint32_t** sptr = reinterpret_cast<const uint32_t**>(sq + 4 * padded);  // column pointers
+  uint32_t total = 0;  // steps of eight entries of all batches
+  for (uint32_t b = 0; b < n_batches; ++b) {
+    const uint32_t first = batches[b].first, count = batches[b].count, room = (count + 7) / 8 * 8;
+    for (uint32_t i = threadIdx.x; i < room; i += MMA_THREADS) {
+      const uint32_t e = first + (i < count ? i : 0);
+      put_reversed(sq + 4 * (8 * total + i), i < count ? coeff_c[e] : qzero());
+      sptr[8 * total + i] = col_ptrs[e];
+    }
+    total += room / 8;
   }
   __syncthreads();
-  const bool aligned = !s_bad;
-  auto load = [&](const uint32_t* p) { return aligned ? V::load(p) : V::load_words(p); };
-  const uint32_t groups = (1u << log_size) / R;
+  const uint32_t lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const mmadot::LaneShifts shifts = mmadot::lane_shifts(g & 1);
+  const uint32_t n_blocks = (1u << log_size) / MMA_ROWS, warps = gridDim.x * (MMA_THREADS / 32);
+  const uint32_t first_blk = blockIdx.x * (MMA_THREADS / 32) + (threadIdx.x >> 5);
   const CircleDomain dom = canonic_domain(log_size);
-  for (uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x; gi < groups; gi += gridDim.x * blockDim.x) {
-    const uint32_t row0 = gi * R;
-    PointM dp[R];
+  WordRing<QUOT_STAGES> ring(qmma);
+  uint32_t p_blk = first_blk, p_step = 0;  // next step to load
+  auto fetch = [&]() {
+    if (p_blk < n_blocks && total) {
+      const uint32_t* const* ptr = sptr + 8 * p_step + ring.column();
 #pragma unroll
-    for (int j = 0; j < R; ++j) dp[j] = pts.at(dom.index_at(bitrev(row0 + j, log_size)));
-    QM31 acc[R];
-#pragma unroll
-    for (int j = 0; j < R; ++j) acc[j] = qzero();
-    for (uint32_t b = 0; b < n_batches; ++b) {
-      const QuotientBatchDev bt = batches[b];
-      uint64_t a[R][4];
-#pragma unroll
-      for (int j = 0; j < R; ++j)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) a[j][c] = 0;
-      auto step = [&](const V& v, const uint4& q) {
-#pragma unroll
-        for (int j = 0; j < R; ++j) {
-          uint32_t vj = v[j];
-          a[j][0] += (uint64_t)q.x * vj;
-          a[j][1] += (uint64_t)q.y * vj;
-          a[j][2] += (uint64_t)q.z * vj;
-          a[j][3] += (uint64_t)q.w * vj;
-        }
-      };
-      auto fold = [&]() {
-#pragma unroll
-        for (int j = 0; j < R; ++j)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) a[j][c] = mfold64(a[j][c]);
-      };
-      uint32_t i = 0;
-      const uint32_t e0 = bt.first;
-      for (; i + U <= bt.count; i += U) {
-        V v[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) v[u] = load(sptr[e0 + i + u] + row0);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          step(v[u], sqe[e0 + i + u]);
-          if (u % 3 == 2) fold();
-        }
-      }
-      for (uint32_t t = 0; i < bt.count; ++i, ++t) {
-        step(load(sptr[e0 + i] + row0), sqe[e0 + i]);
-        if (t % 3 == 2) fold();
-      }
-      quot_batch_finish<R>(bt, dp, a, acc);
+      for (int u = 0; u < 4; ++u) ring.fetch<ALIGNED>(u, ptr[2 * u] + MMA_ROWS * p_blk + ring.row());
+      if (++p_step == total) { p_step = 0; p_blk += warps; }
     }
-    uint32_t w[R];
+    ring.commit();
+  };
+  for (int d = 0; d < QUOT_STAGES; ++d) fetch();
+  for (uint32_t blk = first_blk; blk < n_blocks; blk += warps) {
+    const uint32_t row0 = MMA_ROWS * blk + 2 * g;
+    uint32_t num[4][2] = {};  // this lane's coordinate of the eight rows
+    // The point of the even row of tile t (the odd row's is its conjugate), added up after the loop.
+    const uint32_t idx = dom.index_at(bitrev(row0 + 16 * t, log_size));
+    const PointM plo = pts.lo(idx), phi = pts.hi(idx);
+    const uint32_t* q = sq + 4 * t + (g >> 1);
+    for (uint32_t b = 0; b < n_batches; ++b) {
+      mmadot::Acc acc;
+      acc.clear();
+      for (uint32_t s = (batches[b].count + 7) / 8; s > 0; --s, q += 32) {
+        mmadot::Words w;
+        ring.take(w);
+        acc.step(w, q[0], q[16], shifts);
+        fetch();
+      }
+      const PointM at = padd(plo, phi);
+      CM31 inv[2];
+      {
+        const PointQ pq = batches[b].point;
+        // (Re Px - x) Im Py - (Re Py - y) Im Px at (x, y) and (x, -y).
+        const CM31 u = cmul(csub(pq.x.c0, CM31{at.x, 0}), pq.y.c1);
+        const CM31 den0 = csub(u, cmul(csub(pq.y.c0, CM31{at.y, 0}), pq.x.c1));
+        const CM31 den1 = csub(u, cmul(cadd(pq.y.c0, CM31{at.y, 0}), pq.x.c1));
+        const CM31 both = cmul(den0, den1);
+        if (both.a == 0 && both.b == 0) {  // a zero denominator gives a zero quotient term
+          inv[0] = cinv(den0);
+          inv[1] = cinv(den1);
+        } else {
+          const CM31 r = cinv(both);
+          inv[0] = cmul(r, den1);
+          inv[1] = cmul(r, den0);
+        }
+        __syncwarp();
+      }
+      const uint32_t sum_a = reinterpret_cast<const uint32_t*>(&batches[b].sum_a)[t];
+      const uint32_t sum_b = reinterpret_cast<const uint32_t*>(&batches[b].sum_b)[t];
 #pragma unroll
-    for (int j = 0; j < R; ++j) w[j] = acc[j].c0.a;
-    V::store(out + row0, w);
+      for (int m = 0; m < 4; ++m) {
+        const uint32_t ay = mmul(sum_a, __shfl_sync(0xffffffffu, at.y, m, 4));
 #pragma unroll
-    for (int j = 0; j < R; ++j) w[j] = acc[j].c0.b;
-    V::store(out + out_stride + row0, w);
+        for (int s = 0; s < 2; ++s) {
+          const CM31 iv = {__shfl_sync(0xffffffffu, inv[s].a, m, 4), __shfl_sync(0xffffffffu, inv[s].b, m, 4)};
+          const uint32_t line = s ? msub(sum_b, ay) : madd(sum_b, ay);
+          const uint32_t v = msub(mmadot::row_sum(acc, m, s), line);
+          // (v0 + v1 i)(a + b i): lane t holds v0 (even) or v1 (odd) of its half and keeps that coordinate.
+          const uint32_t o = __shfl_xor_sync(0xffffffffu, v, 1);
+          const uint32_t va = mmul(v, iv.a), ob = mmul(o, iv.b);
+          num[m][s] = madd(num[m][s], t & 1 ? madd(va, ob) : msub(va, ob));
+        }
+      }
+    }
 #pragma unroll
-    for (int j = 0; j < R; ++j) w[j] = acc[j].c1.a;
-    V::store(out + 2 * out_stride + row0, w);
-#pragma unroll
-    for (int j = 0; j < R; ++j) w[j] = acc[j].c1.b;
-    V::store(out + 3 * out_stride + row0, w);
+    for (int m = 0; m < 4; ++m)
+      store_rows2<ALIGNED>(out + t * out_stride + row0 + 16 * m, make_uint2(num[m][0], num[m][1]));
   }
 }
 
@@ -534,7 +599,6 @@ constexpr uint64_t QB_WAIT_NS = 1000000000ull;
 // on that stage runs out.
 std::atomic<bool> g_quot_skip_first_item{false};
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ uint64_t global_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -839,20 +903,28 @@ cudaError_t wide_fib_trace(uint32_t log_n, uint32_t W, int kind, uint64_t seed, 
 cudaError_t wide_fib_composition(uint32_t log_n, uint32_t W, const uint32_t* eval, uint64_t stride,
                                  const QM31* coeffs_dev, uint32_t den_inv0, uint32_t den_inv1, uint32_t* out,
                                  uint64_t out_stride, cudaStream_t stream) {
-  size_t smem = (size_t)(W - 2) * 16;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_composition, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  const bool vec = ((reinterpret_cast<uintptr_t>(eval) | reinterpret_cast<uintptr_t>(out)) & (4 * COMP_R - 1)) == 0 &&
-                   stride % COMP_R == 0 && out_stride % COMP_R == 0 && (2ull << log_n) >= COMP_R;
-  if (vec) {
-    k_composition_v<COMP_R, COMP_U><<<grid_for(2ull << log_n, 256 * COMP_R), 256, smem, stream>>>(
-        log_n, W, eval, stride, coeffs_dev, den_inv0, den_inv1, out, out_stride);
-  } else {
+  const size_t smem = (size_t)(W - 2) * 16;
+  if ((2u << log_n) < MMA_ROWS) {
     k_composition<<<grid_for(2ull << log_n, 256), 256, smem, stream>>>(log_n, W, eval, stride, coeffs_dev, den_inv0,
                                                                        den_inv1, out, out_stride);
+    note_launch();
+    return cudaGetLastError();
   }
+  const bool aligned = ((reinterpret_cast<uintptr_t>(eval) | reinterpret_cast<uintptr_t>(out)) & 15) == 0 &&
+                       stride % 4 == 0 && out_stride % 4 == 0;
+  // Persistent: four CTAs per SM (fewer where W's coefficients fill the shared memory), 64 rows per warp at a time.
+  const uint32_t blocks = (2u << log_n) / MMA_ROWS, per_cta = MMA_THREADS / 32;
+  const uint32_t grid = std::min<uint32_t>((blocks + per_cta - 1) / per_cta, 148 * 4);
+  const size_t smem_m = (size_t)mma_ring_bytes(COMP_STAGES) + (size_t)((W + 7) / 8) * 8 * 32;
+  auto kernel = aligned ? k_composition_mma<true> : k_composition_mma<false>;
+  static const bool attr = [] {  // once per process (thread-safe static initialisation); W <= 3000
+    constexpr int kMax = (int)mma_ring_bytes(COMP_STAGES) + 3008 * 32;
+    cudaFuncSetAttribute(k_composition_mma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax);
+    cudaFuncSetAttribute(k_composition_mma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax);
+    return true;
+  }();
+  (void)attr;
+  kernel<<<grid, MMA_THREADS, smem_m, stream>>>(log_n, W, eval, stride, coeffs_dev, den_inv0, den_inv1, out, out_stride);
   note_launch();
   return cudaGetLastError();
 }
@@ -913,18 +985,16 @@ cudaError_t eval_at_point(const DeviceTables&, uint32_t log_size, uint32_t n_col
   return cudaGetLastError();
 }
 
-template <int R, int U, int MINB>
-static void quotients_smem_attr(size_t smem_v) {
-  cudaFuncSetAttribute(k_quotients_v<R, U, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_v);
-}
-
 void arm_quotient_stage_timeout_for_testing() { g_quot_skip_first_item.store(true); }
 
 cudaError_t accumulate_quotients(const DeviceTables& t, uint32_t log_size, uint32_t n_batches, uint32_t n_entries,
                                  const QuotientBatchDev* batches, const uint32_t* const* col_ptrs, const QM31* coeff_c,
                                  uint32_t* out, uint64_t out_stride, cudaStream_t stream, uint32_t* status) {
-  size_t smem = QUOT_MAX_ENTRIES * 16;
-  size_t smem_v = QUOT_MAX_ENTRIES * (16 + sizeof(void*));
+  const size_t smem = QUOT_MAX_ENTRIES * 16;
+  // Tensor-core kernel: every batch padded to a multiple of eight entries.
+  const uint32_t padded = n_entries + 7 * n_batches;
+  const size_t smem_m = (size_t)mma_ring_bytes(QUOT_STAGES) + (size_t)padded * (16 + sizeof(void*));
+  constexpr size_t SMEM_M_MAX = 200 * 1024;
   // Bulk-staged kernel: the ring, the coefficients and pointers, and the item table (every batch
   // adds at most one partial group).
   const uint32_t item_cap = (n_entries + QB_GROUP - 1) / QB_GROUP + n_batches;
@@ -935,38 +1005,27 @@ cudaError_t accumulate_quotients(const DeviceTables& t, uint32_t log_size, uint3
                                 (size_t)(QUOT_MAX_ENTRIES / QB_GROUP + QB_MAX_BATCHES) * sizeof(QbItem);
   static const bool attr = [&] {  // once per process (thread-safe static initialisation)
     cudaFuncSetAttribute(k_quotients, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    quotients_smem_attr<QUOT_R, QUOT_U, 3>(smem_v);
-    quotients_smem_attr<QUOT_R, 3, 4>(smem_v);
-    quotients_smem_attr<QUOT_R, 9, 2>(smem_v);
+    cudaFuncSetAttribute(k_quotients_mma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_M_MAX);
+    cudaFuncSetAttribute(k_quotients_mma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_M_MAX);
     cudaFuncSetAttribute(k_quotients_bulk<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_B_MAX);
     cudaFuncSetAttribute(k_quotients_bulk<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_B_MAX);
     return true;
   }();
   (void)attr;
-  const bool vec = (reinterpret_cast<uintptr_t>(out) & (4 * QUOT_R - 1)) == 0 && out_stride % QUOT_R == 0 &&
-                   (1ull << log_size) >= QUOT_R;
-  if (!vec) {
+  // The tensor-core kernel takes whole blocks of 64 rows.
+  if ((1ull << log_size) < MMA_ROWS || smem_m > SMEM_M_MAX) {
     k_quotients<<<grid_for(1ull << log_size, 256), 256, smem, stream>>>(PointTable{t.points}, log_size, n_batches,
                                                                         batches, col_ptrs, coeff_c, out, out_stride);
     note_launch();
     return cudaGetLastError();
   }
   // The bulk-staged kernel takes whole 512-row tiles of 16-byte aligned columns (the caller vouches
-  // for the pointers by passing `status`).
+  // for the pointers by passing `status`). It runs when a caller forces the last variant.
   const bool bulk = status != nullptr && log_size >= 16 && n_batches <= QB_MAX_BATCHES &&
                     n_entries <= QUOT_MAX_ENTRIES;
-  // Variants: 6 loads in flight per thread at 3 CTAs per SM, 3 at 4, 9 at 2; bulk-staged.
   auto run = [&](int variant) -> cudaError_t {
-    if (variant == 3 && !bulk) variant = 0;  // a key tuned by a caller that could take it
-    const dim3 grid(grid_for(1ull << log_size, 256 * QUOT_R));
     const PointTable pts{t.points};
-    if (variant == 1)
-      k_quotients_v<QUOT_R, 3, 4><<<grid, 256, smem_v, stream>>>(pts, log_size, n_batches, batches, col_ptrs, coeff_c,
-                                                                   out, out_stride);
-    else if (variant == 2)
-      k_quotients_v<QUOT_R, 9, 2><<<grid, 256, smem_v, stream>>>(pts, log_size, n_batches, batches, col_ptrs, coeff_c,
-                                                                   out, out_stride);
-    else if (variant == 3) {
+    if (variant == 3 && bulk) {
       // Persistent: as many CTAs as stay resident (three per SM while the shared memory allows).
       const int minb = smem_b <= 70 * 1024 ? 3 : 2;
       const uint32_t n_tiles = (uint32_t)((1ull << log_size) / QB_ROWS);
@@ -978,14 +1037,21 @@ cudaError_t accumulate_quotients(const DeviceTables& t, uint32_t log_size, uint3
       else
         k_quotients_bulk<2><<<g, QB_THREADS, smem_b, stream>>>(pts, log_size, n_batches, batches, col_ptrs, coeff_c, n_entries,
                                                         item_cap, out, out_stride, status, skip);
-    } else
-      k_quotients_v<QUOT_R, QUOT_U, 3><<<grid, 256, smem_v, stream>>>(pts, log_size, n_batches, batches, col_ptrs,
-                                                                      coeff_c, out, out_stride);
+    } else {
+      // Persistent: three CTAs per SM, each warp 64 rows at a time. Sixteen-byte copies where the caller
+      // vouches for the columns and the output allows them.
+      const uint32_t blocks = (uint32_t)((1ull << log_size) / MMA_ROWS), per_cta = MMA_THREADS / 32;
+      const uint32_t g = std::min<uint32_t>((blocks + per_cta - 1) / per_cta, t.sm_count * 3);
+      const bool aligned = status != nullptr && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && out_stride % 4 == 0;
+      (aligned ? k_quotients_mma<true> : k_quotients_mma<false>)<<<g, MMA_THREADS, smem_m, stream>>>(
+          pts, log_size, n_batches, batches, col_ptrs, coeff_c, padded, out, out_stride);
+    }
     note_launch();
     return cudaGetLastError();
   };
-  // Reads the columns, writes `out`: re-runnable. Keyed by the committed columns read per row.
-  return tuned_run(TUNE_QUOTIENTS, log_size, n_entries, log_size >= 16 ? (bulk ? 4 : 3) : 1, true, stream, run);
+  // The tensor-core kernel is the fastest variant at every size, so nothing is tuned: variants 1 and 2
+  // are the same kernel, the last one the bulk-staged kernel when forced.
+  return tuned_run(TUNE_QUOTIENTS, log_size, n_entries, log_size >= 16 ? 4 : 1, false, stream, run);
 }
 
 cudaError_t fold_circle_into_line(const DeviceTables& t, uint32_t src_log, const uint32_t* src, uint64_t src_stride,

@@ -1,8 +1,7 @@
 // Launch-shape autotuner, process-wide and keyed by (op, log_size, n_cols).
 //
 // Some kernels come in variants that write the same bits but differ in speed with the shape: the
-// fused or generic FFT high pass, the Merkle leaf kernel built for 4, 5 or 6 CTAs per SM, the
-// quotient kernel with different loads in flight and occupancy. The first call of a key runs every
+// fused or generic FFT high pass, the Merkle leaf kernel built for 4, 5 or 6 CTAs per SM. The first call of a key runs every
 // variant of its op on that call's own inputs, timed with CUDA events on the call's stream (the
 // best of three interleaved runs each), and records the fastest; every later call of the key runs that variant.
 // An op whose outputs overwrite its inputs (an in-place transform) cannot be re-run and takes its
@@ -19,7 +18,7 @@ namespace sb {
 enum TuneOp : uint32_t {
   TUNE_LDE1 = 0,       // interpolate + blow-up-2 extension of 2^16 .. 2^22 columns: fused, generic high pass
   TUNE_LEAVES = 1,     // Merkle leaf kernel: 5, 6, 4 CTAs per SM
-  TUNE_QUOTIENTS = 2,  // DEEP quotients: 6 loads in flight at 3 CTAs/SM, 3 at 4, 9 at 2; bulk-staged
+  TUNE_QUOTIENTS = 2,  // DEEP quotients: not tuned (tensor-core sums); forced variant 3 is the bulk-staged kernel
   TUNE_OPS = 3,
 };
 constexpr int TUNE_MAX_VARIANTS = 4;

@@ -617,7 +617,7 @@ def arm_quotient_stage_timeout_for_testing() -> None:
 
 
 AUTOTUNE_OPS = {0: "interpolate+extend high pass (fused, generic)", 1: "Merkle leaves (5, 6, 4 CTAs/SM)",
-                2: "DEEP quotients (6, 3, 9 loads in flight; bulk-staged)"}
+                2: "DEEP quotients (tensor-core sums; the last forced variant bulk-staged)"}
 
 
 def autotune_mode(mode: int) -> None:
