@@ -274,10 +274,7 @@ __global__ void __launch_bounds__(MMA_THREADS, 4) k_composition_mma(uint32_t log
 
 // ---------------------------------------------------------------------------
 // OODS evaluation (src/prover/poly/circle/poly.zig:62-230): value = sum_j c_j *
-// prod_{bit b of j} F_b with F_0 = y, F_1 = x, F_b = pi^{b-1}(x). A CTA reduces
-// a chunk of 4096 coefficients: 16 per thread against the subset products of
-// F_0..F_3 (lazy 64-bit sums), then two radix-16 levels with F_4..F_7 and
-// F_8..F_11, times the chunk's product of F_12.. .
+// prod_{bit b of j} F_b with F_0 = y, F_1 = x, F_b = pi^{b-1}(x).
 // ---------------------------------------------------------------------------
 constexpr uint32_t OODS_CHUNK_BITS = 12;
 constexpr uint32_t OODS_THREADS = 256;
@@ -291,83 +288,36 @@ __device__ QM31 subset_product(const OodsFactors& F, uint32_t bits, uint32_t fir
   return r;
 }
 
-// A CTA owns one column and a strided set of its 4096-coefficient chunks: chunk = blockIdx.x +
-// k * gridDim.x with gridDim.x a power of two, so a chunk's product of F_12.. splits over disjoint
-// bits into the CTA's part (the bits of blockIdx.x, multiplied in once at the end) and k's part
-// (a table hk[k] in shared memory, each entry a direct product computed by one thread: one barrier).
-// Thread t sums its 16 coefficients of a chunk against the subset products of F_0..F_3, multiplies
-// by hk[k] and accumulates; at the end it multiplies by the CTA's factor and its own (F_4..F_11
-// subset selected by t), and the CTA reduces with warp shuffles to one partial.
-constexpr uint32_t OODS_SMEM_CHUNKS = 1024;  // per-CTA chunk-factor table entries kept in shared memory
-
 __device__ __forceinline__ QM31 shfl_down_q(QM31 v, int d) {
   return qmake(__shfl_down_sync(0xffffffffu, v.c0.a, d), __shfl_down_sync(0xffffffffu, v.c0.b, d),
                __shfl_down_sync(0xffffffffu, v.c1.a, d), __shfl_down_sync(0xffffffffu, v.c1.b, d));
 }
 
-__global__ void __launch_bounds__(OODS_THREADS) k_oods_chunks(OodsFactors F, const uint32_t* __restrict__ coeffs,
-                                                              uint64_t stride, QM31* partial, uint32_t n_chunks) {
+// Columns of fewer than 2^12 coefficients: one CTA a column, thread t sums its 16 coefficients against
+// the subset products of F_0..F_3 and multiplies by its own (F_4.. by the bits of t).
+__global__ void __launch_bounds__(OODS_THREADS) k_oods_small(OodsFactors F, const uint32_t* __restrict__ coeffs,
+                                                             uint64_t stride, QM31* out) {
   __shared__ QM31 b4[3][16];
-  __shared__ QM31 hk[OODS_SMEM_CHUNKS];
   __shared__ QM31 wsum[OODS_THREADS / 32];
-  const uint32_t col = blockIdx.y;
-  const uint32_t L = F.log_size;
-  const uint32_t chunk_bits = L < OODS_CHUNK_BITS ? L : OODS_CHUNK_BITS;
-  const uint32_t g_bits = __ffs(gridDim.x) - 1;  // gridDim.x = 2^g_bits
-  const uint32_t k_first = chunk_bits + g_bits;   // factor index of k's bit 0
-  if (threadIdx.x < 48) {
-    uint32_t lvl = threadIdx.x / 16, r = threadIdx.x % 16;
+  const uint32_t col = blockIdx.x, log = F.log_size, t = threadIdx.x;
+  if (t < 48) {
+    const uint32_t lvl = t / 16, r = t % 16, first = 4 * lvl;
     // factors beyond log_size do not exist; mask them out
-    uint32_t first = 4 * lvl;
-    uint32_t valid_bits = first >= chunk_bits ? 0 : (chunk_bits - first >= 4 ? 4 : chunk_bits - first);
+    const uint32_t valid_bits = first >= log ? 0 : (log - first >= 4 ? 4 : log - first);
     b4[lvl][r] = (r >> valid_bits) ? qzero() : subset_product(F, r, first);
   }
-  const uint32_t n_k = blockIdx.x < n_chunks ? (n_chunks - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-  const uint32_t n_tab = n_k < OODS_SMEM_CHUNKS ? n_k : OODS_SMEM_CHUNKS;
-  for (uint32_t k = threadIdx.x; k < n_tab; k += blockDim.x) hk[k] = subset_product(F, k, k_first);
   __syncthreads();
-  const uint32_t n_in = 1u << chunk_bits;
-  const uint32_t t = threadIdx.x;
-  const bool active = 16 * t < n_in;
-  const uint32_t nw = active ? (n_in - 16 * t < 16 ? n_in - 16 * t : 16) : 0;
-  QM31 acc = qzero();
-  for (uint32_t k = 0; k < n_k && active; ++k) {
-    const uint32_t chunk = blockIdx.x + k * gridDim.x;
-    const uint32_t* c = coeffs + col * stride + ((uint64_t)chunk << chunk_bits) + 16 * t;
-    uint32_t w[16];
-    if (nw == 16) {
-      const uint4* c4 = reinterpret_cast<const uint4*>(c);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint4 x = __ldg(c4 + q);
-        w[4 * q] = x.x; w[4 * q + 1] = x.y; w[4 * q + 2] = x.z; w[4 * q + 3] = x.w;
-      }
-    } else {
-      for (uint32_t r = 0; r < 16; ++r) w[r] = r < nw ? c[r] : 0u;
-    }
-    uint64_t a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-#pragma unroll
-    for (int r = 0; r < 16; ++r) {
-      QM31 bb = b4[0][r];
-      a0 += (uint64_t)bb.c0.a * w[r]; a1 += (uint64_t)bb.c0.b * w[r];
-      a2 += (uint64_t)bb.c1.a * w[r]; a3 += (uint64_t)bb.c1.b * w[r];
-      if (r % 3 == 2) { a0 = mfold64(a0); a1 = mfold64(a1); a2 = mfold64(a2); a3 = mfold64(a3); }
-    }
-    QM31 v = qmake(mreduce64(a0), mreduce64(a1), mreduce64(a2), mreduce64(a3));
-    QM31 h;
-    if (k < OODS_SMEM_CHUNKS) {
-      h = hk[k];
-    } else {  // beyond the table: its low bits from the table, the rest multiplied in
-      h = hk[k & (OODS_SMEM_CHUNKS - 1)];
-      uint32_t bits = k >> 10;
-      for (uint32_t b = k_first + 10; bits; ++b, bits >>= 1)
-        if (bits & 1) h = qmul(h, F.f[b]);
-    }
-    acc = qadd(acc, qmul(v, h));
+  const uint32_t n_in = 1u << log;
+  const uint32_t nw = 16 * t < n_in ? (n_in - 16 * t < 16 ? n_in - 16 * t : 16) : 0;
+  const uint32_t* c = coeffs + col * stride + 16 * t;
+  uint64_t a0 = 0, a1 = 0, a2 = 0, a3 = 0;
+  for (uint32_t r = 0; r < nw; ++r) {
+    const QM31 bb = b4[0][r];
+    const uint32_t w = c[r];
+    a0 = mfold64(a0) + (uint64_t)bb.c0.a * w; a1 = mfold64(a1) + (uint64_t)bb.c0.b * w;
+    a2 = mfold64(a2) + (uint64_t)bb.c1.a * w; a3 = mfold64(a3) + (uint64_t)bb.c1.b * w;
   }
-  // the CTA's factor (bits of blockIdx.x), then the thread's own: subset of F_4..F_7 by bits 0-3
-  // of t, of F_8..F_11 by bits 4-7
-  acc = qmul(acc, subset_product(F, blockIdx.x, chunk_bits));
+  QM31 acc = qmake(mreduce64(a0), mreduce64(a1), mreduce64(a2), mreduce64(a3));
   acc = qmul(acc, qmul(b4[1][t & 15], b4[2][t >> 4]));
 #pragma unroll
   for (int d = 16; d >= 1; d >>= 1) acc = qadd(acc, shfl_down_q(acc, d));
@@ -376,6 +326,97 @@ __global__ void __launch_bounds__(OODS_THREADS) k_oods_chunks(OodsFactors F, con
   if (t == 0) {
     QM31 sum = qzero();
     for (int i = 0; i < OODS_THREADS / 32; ++i) sum = qadd(sum, wsum[i]);
+    out[col] = sum;
+  }
+}
+
+// Columns of 2^12 coefficients or more, the sums on the tensor cores (mma_dot.cuh's limb products). A warp
+// takes chunks of 4096 coefficients, chunk = w + k G with G the column's warps (a power of two), so that a
+// chunk's product of F_12.. splits over disjoint bits into the warp's part (the bits of w, multiplied in
+// once at the end) and k's part (a table hk[k] in shared memory). In a chunk, the coefficients' bits 4..7
+// are the sixteen rows of a product and the other eight bits (lo = 0..3, h = 8..11) its contraction
+// with F_lo F_h, the same 256 coefficients for every chunk and column: one row of 16 coefficients is 64
+// contiguous bytes, so a lane's 16-byte load holds its operand words of two mma steps, and a step h
+// reads 1 KB in a row. The chunk's sixteen sums are multiplied by hk[k] and accumulated per row; the
+// row's own factor (F_4..F_7) comes at the end.
+// 100 columns of 2^20: 89 us, 4.7 TB/s (16 coefficients a thread with 64-bit multiply-adds: 145 us).
+constexpr uint32_t OODS_SMEM_CHUNKS = 1024;  // chunk-factor table entries kept in shared memory
+constexpr uint32_t OODS_WARPS = 4;
+
+__global__ void __launch_bounds__(32 * OODS_WARPS) k_oods_mma(OodsFactors F, const uint32_t* __restrict__ coeffs,
+                                                              uint64_t stride, QM31* partial, uint32_t n_chunks) {
+  __shared__ QM31 f_lo[16], f_row[16], f_h[16];
+  __shared__ uint32_t tab[16][4][4][4];  // [h][lo & 3][lo >> 2][coordinate], byte-reversed
+  __shared__ QM31 hk[OODS_SMEM_CHUNKS];
+  __shared__ QM31 wsum[OODS_WARPS];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, col = blockIdx.y;
+  const uint32_t n_warps = gridDim.x * OODS_WARPS, w = blockIdx.x * OODS_WARPS + warp;
+  const uint32_t k_first = OODS_CHUNK_BITS + __ffs(n_warps) - 1;  // factor index of k's bit 0
+  if (threadIdx.x < 48) {
+    const uint32_t lvl = threadIdx.x / 16, r = threadIdx.x % 16;
+    (lvl == 0 ? f_lo : lvl == 1 ? f_row : f_h)[r] = subset_product(F, r, 4 * lvl);
+  }
+  const uint32_t n_k = (n_chunks + n_warps - 1) / n_warps;  // of the CTA's first warp, the most
+  for (uint32_t k = threadIdx.x; k < n_k && k < OODS_SMEM_CHUNKS; k += 32 * OODS_WARPS) hk[k] = subset_product(F, k, k_first);
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < 256; i += 32 * OODS_WARPS)
+    put_reversed(tab[i >> 4][i & 3][(i >> 2) & 3], qmul(f_lo[i & 15], f_h[i >> 4]));
+  __syncthreads();
+  const mmadot::LaneShifts shifts = mmadot::lane_shifts(g & 1);
+  const uint32_t* b = &tab[0][0][t][g >> 1];
+  QM31 acc = qzero();  // lanes t = 0 and 1: rows g and g + 8
+  for (uint32_t k = 0, chunk = w; chunk < n_chunks; ++k, chunk += n_warps) {
+    const uint4* c = reinterpret_cast<const uint4*>(coeffs + col * stride + ((uint64_t)chunk << OODS_CHUNK_BITS)) + lane;
+    int32_t s[4][4];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) s[i >> 2][i & 3] = 0;
+    constexpr int HALF = 8;  // h steps loaded together: 16 KB in flight per CTA
+#pragma unroll 1
+    for (int h0 = 0; h0 < 16; h0 += HALF) {
+      uint4 x[HALF], y[HALF];
+#pragma unroll
+      for (int h = 0; h < HALF; ++h) {
+        x[h] = __ldg(c + (h0 + h) * 64);
+        y[h] = __ldg(c + (h0 + h) * 64 + 32);
+      }
+#pragma unroll
+      for (int h = 0; h < HALF; ++h) {
+        const uint32_t* bh = b + (h0 + h) * 64;
+        uint32_t e0[4], e1[4];
+        mmadot::expand(bh[0], shifts, e0);
+        mmadot::expand(bh[16], shifts, e1);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) mmadot::mma_u8(s[i], x[h].x, y[h].x, x[h].y, y[h].y, e0[i], e1[i]);
+        mmadot::expand(bh[32], shifts, e0);
+        mmadot::expand(bh[48], shifts, e1);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) mmadot::mma_u8(s[i], x[h].z, y[h].z, x[h].w, y[h].w, e0[i], e1[i]);
+      }
+    }
+    const uint32_t v0 = mmadot::combine(s, 0), v1 = mmadot::combine(s, 1);
+    uint32_t v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t a = __shfl_sync(0xffffffffu, v0, j, 4), d = __shfl_sync(0xffffffffu, v1, j, 4);
+      v[j] = t & 1 ? d : a;
+    }
+    QM31 f = hk[k & (OODS_SMEM_CHUNKS - 1)];
+    if (k >= OODS_SMEM_CHUNKS) {  // beyond the table: the rest of k's bits multiplied in
+      uint32_t bits = k / OODS_SMEM_CHUNKS;
+      for (uint32_t i = k_first + 10; bits; ++i, bits >>= 1)
+        if (bits & 1) f = qmul(f, F.f[i]);
+    }
+    acc = qadd(acc, qmul(qload4(v), f));
+  }
+  acc = t < 2 ? qmul(acc, qmul(f_row[g + 8 * t], subset_product(F, w, OODS_CHUNK_BITS))) : qzero();
+  __syncwarp();
+#pragma unroll
+  for (int d = 16; d >= 1; d >>= 1) acc = qadd(acc, shfl_down_q(acc, d));
+  if (lane == 0) wsum[warp] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    QM31 sum = qzero();
+    for (uint32_t i = 0; i < OODS_WARPS; ++i) sum = qadd(sum, wsum[i]);
     partial[(uint64_t)col * gridDim.x + blockIdx.x] = sum;
   }
 }
@@ -971,14 +1012,16 @@ cudaError_t eval_at_point(const DeviceTables&, uint32_t log_size, uint32_t n_col
     QM31 x = p.x;
     for (uint32_t b = 1; b < log_size; ++b) { F.f[b] = x; x = qdouble_x(x); }
   }
-  uint32_t chunk_bits = log_size < OODS_CHUNK_BITS ? log_size : OODS_CHUNK_BITS;
-  uint32_t n_chunks = 1u << (log_size - chunk_bits);
-  // A power of two of CTAs per column (the chunk factor splits over the CTA's bits): about four
-  // waves of five CTAs per SM over all columns, never more CTAs per column than chunks.
+  if (log_size < OODS_CHUNK_BITS) {
+    k_oods_small<<<n_cols, OODS_THREADS, 0, stream>>>(F, coeffs, stride, out); note_launch();
+    return cudaGetLastError();
+  }
+  const uint32_t n_chunks = 1u << (log_size - OODS_CHUNK_BITS);
+  // A power of two of CTAs per column (the chunk factor splits over the warp's bits): about twenty CTAs of
+  // four warps per SM over all columns, no more than give every warp a chunk.
   uint32_t per_col = 1;
-  while (per_col < n_chunks && (uint64_t)per_col * n_cols < 148ull * 5 * 4) per_col <<= 1;
-  dim3 grid(per_col, n_cols);
-  k_oods_chunks<<<grid, OODS_THREADS, 0, stream>>>(F, coeffs, stride, partial, n_chunks); note_launch();
+  while (per_col * OODS_WARPS < n_chunks && (uint64_t)per_col * n_cols < 148ull * 20) per_col <<= 1;
+  k_oods_mma<<<dim3(per_col, n_cols), 32 * OODS_WARPS, 0, stream>>>(F, coeffs, stride, partial, n_chunks); note_launch();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   k_oods_sum<<<(n_cols + 3) / 4, 128, 0, stream>>>(partial, per_col, n_cols, out); note_launch();
