@@ -212,7 +212,8 @@ __global__ void k_fft_high(HighParams p) {
   }
 }
 
-// Entries 2^R .. 2^(R+1) of tw and itw are the doubled copies (tw2, itw2).
+// Entries 2^R .. 2^(R+1) of tw and itw are the doubled balanced copies (tw2, itw2; fft16.cuh).
+__device__ __forceinline__ uint32_t doubled(uint32_t t) { return 2 * (t > P / 2 ? t - P : t); }
 __global__ void k_build_tower(PointTable pts, uint32_t R, uint32_t* tw, uint32_t* itw) {
   // Entry e < 2^R - 1 belongs to layer k with offset 2^R - 2^(R-k).
   uint64_t total = 1ull << R;
@@ -230,8 +231,8 @@ __global__ void k_build_tower(PointTable pts, uint32_t R, uint32_t* tw, uint32_t
     const uint32_t ix = minv(x);
     tw[e] = x;
     itw[e] = ix;
-    tw[total + e] = 2 * x;
-    itw[total + e] = 2 * ix;
+    tw[total + e] = doubled(x);
+    itw[total + e] = doubled(ix);
   }
 }
 
@@ -257,7 +258,8 @@ __device__ __forceinline__ void exchange12(uint32_t* sm, uint32_t (&x)[16], uint
   for (int k = 0; k < 16; ++k) x[k] = sm[b ^ swz((uint32_t)k << WB)];
 }
 
-// Layers 0..11 of blocks of 4096 words. Forward: windows [8,12) -> [4,8) -> [0,4);
+// Layers 0..11 of blocks of 4096 words. Forward: windows [8,12) -> [4,8) -> [0,4), from S words
+// (fft16.cuh; the high pass leaves them, canonical words are also S) to canonical ones;
 // inverse: the reverse, then the optional scale.
 // With TMA (forward only) the block leaves through shared memory: each thread writes its 16 words
 // as four 16-byte vectors into the 128-byte swizzled layout of `out_map` (rows of 32 words, the
@@ -288,7 +290,7 @@ __global__ void __launch_bounds__(256) k_fft_low12(const uint32_t* __restrict__ 
     radix16<false, 0, 4>(x, tv, 0, 4, blk + ib1);
     __syncthreads();
     exchange12<4, 0>(sm, x, ib1, ib0);
-    radix16<false, 0, 4>(x, tv, 0, 0, blk + ib0);
+    radix16<false, 0, 4, fft16::RANGE_S, fft16::RANGE_CANON>(x, tv, 0, 0, blk + ib0);
     // The swizzled layout assumes a 1024-byte aligned buffer (the alignment declared above); a
     // buffer placed otherwise takes the plain stores.
     if (TMA && (((uint32_t)__cvta_generic_to_shared(sm)) & 1023u) == 0) {
@@ -551,8 +553,8 @@ __global__ void __launch_bounds__(1 << R, R <= 8 ? (1024 >> R) : 1) k_fft_high16
       x[k] = v;
       y[k] = v;
     }
-    radix16<false, 0, 4>(x, p.ftv, B12, w0, mb);
-    radix16<false, 0, 4>(y, p.ftv, B12, w0, mb | (1u << R));
+    radix16<false, 0, 4, fft16::RANGE_CANON>(x, p.ftv, B12, w0, mb);
+    radix16<false, 0, 4, fft16::RANGE_CANON>(y, p.ftv, B12, w0, mb | (1u << R));
     const uint32_t a = swz((mb << 4) | t);
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
