@@ -419,14 +419,18 @@ int32_t WideFibProver::prove(const ProveRequest& req, std::string& out, StageTim
   PointQ oods = random_secure_point(ch);
   gap_end();
   SB_CK(eval_at_point(T, n, W, b.coeffs, l.N, oods, nullptr, b.oods_partial, b.oods_out, fs));
-  SB_CK(eval_at_point(T, n, 4, b.comp, l.NC, oods, nullptr, b.oods_partial, b.oods_out + W, fs));
-  SB_CK(eval_at_point(T, n, 4, b.comp + l.N, l.NC, oods, nullptr, b.oods_partial, b.oods_out + W + 4, fs));
+  // The composition's halves are eight columns 2^n words apart: coordinate c's left half, then its right.
+  SB_CK(eval_at_point(T, n, 8, b.comp, l.N, oods, nullptr, b.oods_partial, b.oods_out + W, fs));
   std::vector<QM31> sampled(W + 8);
   SB_CK(cudaMemcpyAsync(pin, b.oods_out, (W + 8) * sizeof(QM31), cudaMemcpyDeviceToHost, fs));
   SB_CK(cudaEventRecord(ev_[6], fs));
   SB_CK(fsync());
   gap = Clock::now();
-  std::memcpy(sampled.data(), pin, (W + 8) * sizeof(QM31));
+  {
+    const QM31* v = reinterpret_cast<const QM31*>(pin);
+    std::copy(v, v + W, sampled.begin());
+    for (uint32_t c = 0; c < 8; ++c) sampled[W + c] = v[W + 2 * (c & 3) + (c >> 2)];  // left halves, then right
+  }
   ch.mix_felts(sampled.data(), sampled.size());
   QM31 quot_coeff = ch.draw_secure_felt();
 

@@ -338,11 +338,14 @@ __global__ void __launch_bounds__(OODS_THREADS) k_oods_small(OodsFactors F, cons
 // with F_lo F_h, the same 256 coefficients for every chunk and column: one row of 16 coefficients is 64
 // contiguous bytes, so a lane's 16-byte load holds its operand words of two mma steps, and a step h
 // reads 1 KB in a row. The chunk's sixteen sums are multiplied by hk[k] and accumulated per row; the
-// row's own factor (F_4..F_7) comes at the end.
+// row's own factor (F_4..F_7) comes at the end. HN: the steps of a chunk that one warp takes. All sixteen
+// when there are chunks for every scheduler; otherwise four warps share a chunk (four columns of 2^18:
+// 13 us with whole chunks, 6.2 us with quarters).
 // 100 columns of 2^20: 89 us, 4.7 TB/s (16 coefficients a thread with 64-bit multiply-adds: 145 us).
 constexpr uint32_t OODS_SMEM_CHUNKS = 1024;  // chunk-factor table entries kept in shared memory
 constexpr uint32_t OODS_WARPS = 4;
 
+template <int HN>
 __global__ void __launch_bounds__(32 * OODS_WARPS) k_oods_mma(OodsFactors F, const uint32_t* __restrict__ coeffs,
                                                               uint64_t stride, QM31* partial, uint32_t n_chunks) {
   __shared__ QM31 f_lo[16], f_row[16], f_h[16];
@@ -350,7 +353,9 @@ __global__ void __launch_bounds__(32 * OODS_WARPS) k_oods_mma(OodsFactors F, con
   __shared__ QM31 hk[OODS_SMEM_CHUNKS];
   __shared__ QM31 wsum[OODS_WARPS];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, col = blockIdx.y;
-  const uint32_t n_warps = gridDim.x * OODS_WARPS, w = blockIdx.x * OODS_WARPS + warp;
+  constexpr uint32_t PARTS = 16 / HN;  // warps per chunk
+  const uint32_t n_warps = gridDim.x * OODS_WARPS / PARTS, unit = blockIdx.x * OODS_WARPS + warp, w = unit / PARTS;
+  const uint32_t h_first = unit % PARTS * HN;
   const uint32_t k_first = OODS_CHUNK_BITS + __ffs(n_warps) - 1;  // factor index of k's bit 0
   if (threadIdx.x < 48) {
     const uint32_t lvl = threadIdx.x / 16, r = threadIdx.x % 16;
@@ -363,16 +368,17 @@ __global__ void __launch_bounds__(32 * OODS_WARPS) k_oods_mma(OodsFactors F, con
     put_reversed(tab[i >> 4][i & 3][(i >> 2) & 3], qmul(f_lo[i & 15], f_h[i >> 4]));
   __syncthreads();
   const mmadot::LaneShifts shifts = mmadot::lane_shifts(g & 1);
-  const uint32_t* b = &tab[0][0][t][g >> 1];
+  const uint32_t* b = &tab[h_first][0][t][g >> 1];
   QM31 acc = qzero();  // lanes t = 0 and 1: rows g and g + 8
   for (uint32_t k = 0, chunk = w; chunk < n_chunks; ++k, chunk += n_warps) {
-    const uint4* c = reinterpret_cast<const uint4*>(coeffs + col * stride + ((uint64_t)chunk << OODS_CHUNK_BITS)) + lane;
+    const uint4* c = reinterpret_cast<const uint4*>(coeffs + col * stride + ((uint64_t)chunk << OODS_CHUNK_BITS)) +
+                     h_first * 64 + lane;
     int32_t s[4][4];
 #pragma unroll
     for (int i = 0; i < 16; ++i) s[i >> 2][i & 3] = 0;
-    constexpr int HALF = 8;  // h steps loaded together: 16 KB in flight per CTA
+    constexpr int HALF = HN < 8 ? HN : 8;  // h steps loaded together
 #pragma unroll 1
-    for (int h0 = 0; h0 < 16; h0 += HALF) {
+    for (int h0 = 0; h0 < HN; h0 += HALF) {
       uint4 x[HALF], y[HALF];
 #pragma unroll
       for (int h = 0; h < HALF; ++h) {
@@ -1018,10 +1024,13 @@ cudaError_t eval_at_point(const DeviceTables&, uint32_t log_size, uint32_t n_col
   }
   const uint32_t n_chunks = 1u << (log_size - OODS_CHUNK_BITS);
   // A power of two of CTAs per column (the chunk factor splits over the warp's bits): about twenty CTAs of
-  // four warps per SM over all columns, no more than give every warp a chunk.
+  // four warps per SM over all columns, no more than give every warp work. Fewer chunks than four warps per
+  // scheduler: a chunk per CTA instead of per warp.
+  const bool quarters = (uint64_t)n_chunks * n_cols < 148ull * 16;
+  const uint32_t per_cta = quarters ? 1 : OODS_WARPS;  // chunks
   uint32_t per_col = 1;
-  while (per_col * OODS_WARPS < n_chunks && (uint64_t)per_col * n_cols < 148ull * 20) per_col <<= 1;
-  k_oods_mma<<<dim3(per_col, n_cols), 32 * OODS_WARPS, 0, stream>>>(F, coeffs, stride, partial, n_chunks); note_launch();
+  while (per_col * per_cta < n_chunks && (uint64_t)per_col * n_cols < 148ull * 20) per_col <<= 1;
+  (quarters ? k_oods_mma<4> : k_oods_mma<16>)<<<dim3(per_col, n_cols), 32 * OODS_WARPS, 0, stream>>>(F, coeffs, stride, partial, n_chunks); note_launch();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   k_oods_sum<<<(n_cols + 3) / 4, 128, 0, stream>>>(partial, per_col, n_cols, out); note_launch();

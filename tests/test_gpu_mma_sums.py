@@ -4,6 +4,7 @@ outputs that are not 16-byte aligned; against the definitions in Python integers
 import numpy as np
 import pytest
 
+import oracle
 import verifier as V
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +66,18 @@ def test_quotients(ctx, log, n, offset):
         num = V.qsub(num, V.qadd(V.qmulm(sa, y), sb))
         den = V.csub(V.cmul(V.csub(px[0], (x, 0)), py[1]), V.cmul(V.csub(py[0], (y, 0)), px[1]))
         assert got[:, row].tolist() == list(V.qflat(V.qmulc(num, V.cinv(den)))), row
+
+
+@pytest.mark.parametrize("log,n", [(0, 3), (3, 2), (11, 5), (12, 1), (13, 33), (14, 600), (16, 160), (18, 38)])
+def test_openings(ctx, log, n):
+    """Below the tensor-core kernel's 2^12, with a chunk per warp and per CTA, several chunks a warp."""
+    import torch
+    rng = np.random.default_rng(log)
+    cols = rng.integers(0, P, size=(n, 1 << log), dtype=np.uint32)
+    cols[0] = P - 1
+    px, py = rng.integers(0, P, size=(2, 4)).tolist()
+    out = torch.empty(4 * n, dtype=torch.int32, device="cuda")
+    ctx.eval_at_point(_dev(cols, 0), log, n, 1 << log, px, py, out)
+    got = _words(out).reshape(n, 4)
+    for c in {0, n // 2, n - 1}:
+        assert np.array_equal(got[c], oracle.eval_at_point(cols[c], px, py)), c
