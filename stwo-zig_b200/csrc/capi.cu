@@ -494,13 +494,14 @@ int32_t stwo_b200_pow_grind(stwo_b200_context* ctx, const uint8_t prefix_digest[
   uint32_t* res = ctx->ctx.small;
   uint32_t w[8];
   std::memcpy(w, prefix_digest, 32);
-  // The prover's search: bounded rounds in nonce order, four per check, at most 2^(bits+16) nonces.
+  // The prover's search: bounded rounds in nonce order, up to four per check, at most 2^(bits+16) nonces.
   const uint64_t max_nonce = n_bits >= 48 ? ~0ull : (1ull << (n_bits + 16));
-  const uint64_t per_round = sb::pow_round_nonces(ctx->ctx.sm_count);
+  const uint64_t per_round = sb::pow_round_nonces(ctx->ctx.sm_count, n_bits);
+  const uint32_t per_check = sb::pow_rounds_per_check(ctx->ctx.sm_count, n_bits);
   cudaError_t e = cudaMemsetAsync(res, 0xff, 8, s);
   uint64_t nonce = ~0ull;
   for (uint64_t base = 0; e == cudaSuccess && base < max_nonce && nonce == ~0ull;) {
-    for (int r = 0; r < 4 && base < max_nonce && e == cudaSuccess; ++r, base += per_round)
+    for (uint32_t r = 0; r < per_check && base < max_nonce && e == cudaSuccess; ++r, base += per_round)
       e = sb::pow_round(w, n_bits, base, res, ctx->ctx.sm_count, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&nonce, res, 8, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

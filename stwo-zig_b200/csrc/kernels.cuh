@@ -163,8 +163,10 @@ cudaError_t fri_tail(const DeviceTables& t, FriChannelDev* c, uint32_t L, uint32
 // ---- Proof of work (src/core/channel/blake2s.zig:135-240) ------------------
 // Bounded rounds of the same search (the form the prover uses, so the grind
 // never holds every SM slot for the whole search): result_dev[0..1] must start
-// at ~0; round r covers nonces [base, base + pow_round_nonces(sm_count)).
-uint64_t pow_round_nonces(int sm_count);
+// at ~0; a round covers nonces [base, base + pow_round_nonces(sm_count, n_bits)), and
+// pow_rounds_per_check rounds are enqueued before the result is read back.
+uint64_t pow_round_nonces(int sm_count, uint32_t n_bits);
+uint32_t pow_rounds_per_check(int sm_count, uint32_t n_bits);
 cudaError_t pow_round(const uint32_t prefix_words[8], uint32_t n_bits, uint64_t base, uint32_t* result_dev,
                       int sm_count, cudaStream_t stream);
 

@@ -14,6 +14,7 @@
 // rest by one launch of k_merkle_top.
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <utility>
 
 #include "blake2s.cuh"
@@ -953,23 +954,42 @@ __global__ void __launch_bounds__(256) k_pow_round(PowPrefix pre, uint32_t n_bit
 
 }  // namespace
 
-uint64_t pow_round_nonces(int sm_count) { return (uint64_t)sm_count * 4 * 256 * 112; }
+namespace {
+struct PowShape { uint32_t grid, per_thread; };
+// A full round: four waves of short CTAs (32 registers: eight 256-thread CTAs resident per SM;
+// 14 nonces per thread, ~0.15 ms a wave) rather than one wave of long ones, so
+// that other streams' work gets SMs between them. An easier target (2^n_bits nonces expected) takes a
+// round of eight times that, which misses with probability e^-8: a full round's grid is launched and
+// drained for nothing (10 bits: 58 us, and 11.5 us for each round enqueued behind it; now one launch of 3.8 us).
+PowShape pow_shape(int sm_count, uint32_t n_bits) {
+  const uint64_t resident = (uint64_t)sm_count * 8 * 256, full = resident * 4 * 14;
+  const uint64_t want = n_bits < 40 ? 8ull << n_bits : full;
+  if (want >= full) return {(uint32_t)sm_count * 4 * 8, 14};
+  const uint32_t per_thread = (uint32_t)std::min<uint64_t>(14, (want + resident - 1) / resident);
+  return {(uint32_t)((want + 256ull * per_thread - 1) / (256ull * per_thread)), per_thread};
+}
+}  // namespace
+
+uint64_t pow_round_nonces(int sm_count, uint32_t n_bits) {
+  const PowShape s = pow_shape(sm_count, n_bits);
+  return (uint64_t)s.grid * 256 * s.per_thread;
+}
+uint32_t pow_rounds_per_check(int sm_count, uint32_t n_bits) {
+  return (8ull << std::min(n_bits, 40u)) > pow_round_nonces(sm_count, n_bits) ? 4 : 1;
+}
 
 cudaError_t pow_round(const uint32_t prefix_words[8], uint32_t n_bits, uint64_t base, uint32_t* result_dev,
                       int sm_count, cudaStream_t stream) {
   const PowPrefix pre = pow_prefix(prefix_words);
-  // Four waves of short CTAs (32 registers: eight 256-thread CTAs resident per SM;
-  // 14 nonces per thread, ~0.15 ms a wave) rather than one wave of long ones, so
-  // that other streams' work gets SMs between them.
   auto* res = reinterpret_cast<unsigned long long*>(result_dev);
-  const bool hi0 = base + pow_round_nonces(sm_count) <= (1ull << 32);
-  const uint32_t grid = sm_count * 4 * 8;
+  const bool hi0 = base + pow_round_nonces(sm_count, n_bits) <= (1ull << 32);
+  const PowShape s = pow_shape(sm_count, n_bits);
   if (n_bits <= 32) {
-    if (hi0) k_pow_round<true, true><<<grid, 256, 0, stream>>>(pre, n_bits, base, 14, res, 1u);
-    else k_pow_round<true, false><<<grid, 256, 0, stream>>>(pre, n_bits, base, 14, res, 1u);
+    if (hi0) k_pow_round<true, true><<<s.grid, 256, 0, stream>>>(pre, n_bits, base, s.per_thread, res, 1u);
+    else k_pow_round<true, false><<<s.grid, 256, 0, stream>>>(pre, n_bits, base, s.per_thread, res, 1u);
   } else {
-    if (hi0) k_pow_round<false, true><<<grid, 256, 0, stream>>>(pre, n_bits, base, 14, res, 1u);
-    else k_pow_round<false, false><<<grid, 256, 0, stream>>>(pre, n_bits, base, 14, res, 1u);
+    if (hi0) k_pow_round<false, true><<<s.grid, 256, 0, stream>>>(pre, n_bits, base, s.per_thread, res, 1u);
+    else k_pow_round<false, false><<<s.grid, 256, 0, stream>>>(pre, n_bits, base, s.per_thread, res, 1u);
   }
   note_launch();
   return cudaGetLastError();

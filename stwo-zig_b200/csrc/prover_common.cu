@@ -126,14 +126,15 @@ int32_t fri_pow_queries(const DeviceTables& T, int sm_count, Channel& ch, const 
     }
     uint32_t pw[8];
     std::memcpy(pw, prefix, 32);
-    // Rounds of ~17M nonces, four per check; the search bound is 2^(bits+16) nonces.
+    // Rounds of up to ~17M nonces, up to four per check; the search bound is 2^(bits+16) nonces.
     const uint64_t max_nonce = cfg.pow_bits >= 48 ? ~0ull : (1ull << (cfg.pow_bits + 16));
-    const uint64_t per_round = pow_round_nonces(sm_count);
+    const uint64_t per_round = pow_round_nonces(sm_count, cfg.pow_bits);
+    const uint32_t per_check = pow_rounds_per_check(sm_count, cfg.pow_bits);
     SB_CKE(cudaMemsetAsync(fb.pow_result, 0xff, 8, s));
     nonce = ~0ull;
     for (uint64_t base = 0; base < max_nonce && nonce == ~0ull;) {
       out.host_gap_ms += std::chrono::duration<float, std::milli>(Clock::now() - out.gap_start).count();
-      for (int r = 0; r < 4 && base < max_nonce; ++r, base += per_round)
+      for (uint32_t r = 0; r < per_check && base < max_nonce; ++r, base += per_round)
         SB_CKE(pow_round(pw, cfg.pow_bits, base, fb.pow_result, sm_count, s));
       SB_CKE(cudaMemcpyAsync(pin, fb.pow_result, 8, cudaMemcpyDeviceToHost, s));
       SB_CKE(stream_wait(s));

@@ -1,6 +1,8 @@
 """The launches that end a tree and the FRI phase (a CTA or a cluster, four lanes per hash): every
 stored node at the sizes where the launches and cluster sizes change, and whole proofs whose FRI tail
-starts at each layer size, with one and with eight CTAs."""
+starts at each layer size, with one and with eight CTAs; the proof-of-work rounds of easy targets."""
+import struct
+
 import numpy as np
 import pytest
 
@@ -27,3 +29,12 @@ def test_fri_tail(ctx, log_n, last):
     g = sb.PcsConfig(o.pow_bits, sb.FriConfig(o.log_blowup_factor, last, o.n_queries))
     got = ctx.prove_wide_fibonacci(sb.Statement(log_n, 5), g, trace_kind=sb.TRACE_SEEDED, trace_seed=log_n)
     assert got == oracle.prove_wide_fib(log_n, 5, o, trace_kind=1, trace_seed=log_n)
+
+
+@pytest.mark.parametrize("bits", [3, 11, 16, 18, 20, 21, 22])
+def test_grind_round_shapes(ctx, bits):
+    """Targets whose rounds have one nonce a thread, several, a full round's grid; the lowest nonce each time."""
+    for i in range(3):
+        digest = bytes((i * 53 + bits + k) & 0xFF for k in range(32))
+        prefix = oracle.blake2s(struct.pack("<I", 0x12345678) + b"\0" * 12 + digest + struct.pack("<I", bits))
+        assert ctx.pow_grind(prefix, bits) == oracle.pow_grind(digest, bits, 8)
