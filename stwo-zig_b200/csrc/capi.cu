@@ -81,6 +81,18 @@ bool domain_ok(const stwo_b200_context* c, uint32_t log_size) {
   return log_size >= 1 && log_size <= c->ctx.tables.tower_log + 1;
 }
 
+int32_t read_root(stwo_b200_context* ctx, uint8_t* root_host, const uint8_t* layers_dev, uint32_t log_size, cudaStream_t s,
+                  const char* what) {
+  if (!root_host) return STWO_B200_OK;
+  const uint64_t root_node = (2ull << log_size) - 2;
+  sb::PinnedSlots::Slot slot(ctx->ctx.slots);  // staged through page-locked memory when one is free
+  uint8_t* to = slot.data() ? slot.data() : root_host;
+  cudaError_t e = cudaMemcpyAsync(to, layers_dev + root_node * 32, 32, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess && to != root_host) std::memcpy(root_host, to, 32);
+  return cuda_status(e, what);
+}
+
 }  // namespace
 
 extern "C" {
@@ -247,13 +259,7 @@ int32_t stwo_b200_merkle_commit(stwo_b200_context* ctx, uint32_t log_size, uint3
   if (n_cols == 0) log_size = 0;
   cudaError_t e = sb::merkle_commit(log_size, n_cols, cols, stride, layers_dev, st(stream));
   if (e != cudaSuccess) return cuda_status(e, "merkle_commit");
-  if (root_host) {
-    uint64_t root_node = (2ull << log_size) - 2;
-    e = cudaMemcpyAsync(root_host, layers_dev + root_node * 32, 32, cudaMemcpyDeviceToHost, st(stream));
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st(stream));
-    return cuda_status(e, "merkle root readback");
-  }
-  return STWO_B200_OK;
+  return read_root(ctx, root_host, layers_dev, log_size, st(stream), "merkle root readback");
 }
 
 int32_t stwo_b200_merkle_commit_lifted(stwo_b200_context* ctx, uint32_t n_cols, const uint32_t* const* cols,
@@ -298,13 +304,7 @@ int32_t stwo_b200_merkle_commit_lifted(stwo_b200_context* ctx, uint32_t n_cols, 
     if (e == cudaSuccess) e = e2;
   }
   if (e != cudaSuccess) return cuda_status(e, "merkle_commit_lifted");
-  if (root_host) {
-    const uint64_t leaves = n_cols ? (1ull << max_log) : 1;
-    e = cudaMemcpyAsync(root_host, layers_dev + (2 * leaves - 2) * 32, 32, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    return cuda_status(e, "merkle root readback");
-  }
-  return STWO_B200_OK;
+  return read_root(ctx, root_host, layers_dev, n_cols ? max_log : 0, s, "merkle root readback");
 }
 
 int32_t stwo_b200_fold_circle_into_line(stwo_b200_context* ctx, uint32_t src_log, const uint32_t* src,
@@ -329,16 +329,6 @@ int32_t stwo_b200_fold_line(stwo_b200_context* ctx, uint32_t src_log, const uint
                      "fold_line");
 }
 
-namespace {
-int32_t read_root(uint8_t* root_host, const uint8_t* layers_dev, uint32_t log_size, cudaStream_t s,
-                  const char* what) {
-  if (!root_host) return STWO_B200_OK;
-  const uint64_t root_node = (2ull << log_size) - 2;
-  cudaError_t e = cudaMemcpyAsync(root_host, layers_dev + root_node * 32, 32, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  return cuda_status(e, what);
-}
-}  // namespace
 
 int32_t stwo_b200_fold_and_commit(stwo_b200_context* ctx, int32_t circle, uint32_t src_log, const uint32_t* src,
                                   uint64_t src_stride, stwo_b200_qm31 alpha, uint32_t* dst, uint64_t dst_stride,
@@ -349,18 +339,10 @@ int32_t stwo_b200_fold_and_commit(stwo_b200_context* ctx, int32_t circle, uint32
       dst_stride < (1ull << (src_log - 1)) || (root_host && !layers_dev) || (layers_dev && !is_aligned(layers_dev, 16)))
     return set_error(STWO_B200_E_INVALID, "bad fold_and_commit arguments");
   cudaStream_t s = st(stream);
-  void* a_dev = nullptr;
-  cudaError_t e = cudaMallocAsync(&a_dev, sizeof(sb::QM31), s);
-  if (e != cudaSuccess) return cuda_status(e, "fold_and_commit alpha");
-  const sb::QM31 a = q(alpha);
-  e = cudaMemcpyAsync(a_dev, &a, sizeof(a), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess)
-    e = sb::fri_fold_commit(ctx->ctx.tables, circle != 0, src_log, src, src_stride,
-                            static_cast<const sb::QM31*>(a_dev), dst, dst_stride, layers_dev, s);
-  cudaError_t e2 = cudaFreeAsync(a_dev, s);
+  const cudaError_t e = sb::fri_fold_commit(ctx->ctx.tables, circle != 0, src_log, src, src_stride, nullptr, dst,
+                                            dst_stride, layers_dev, s, q(alpha));
   if (e != cudaSuccess) return cuda_status(e, "fold_and_commit");
-  if (e2 != cudaSuccess) return cuda_status(e2, "fold_and_commit alpha free");
-  return read_root(root_host, layers_dev, src_log - 1, s, "fold_and_commit root readback");
+  return read_root(ctx, root_host, layers_dev, src_log - 1, s, "fold_and_commit root readback");
 }
 
 int32_t stwo_b200_commit_columns(stwo_b200_context* ctx, uint32_t log_size, uint32_t log_blowup, uint32_t n_cols,
@@ -376,7 +358,7 @@ int32_t stwo_b200_commit_columns(stwo_b200_context* ctx, uint32_t log_size, uint
                                          coeffs_stride, lde, lde_stride, s);
   if (e == cudaSuccess) e = sb::merkle_commit(log_size + log_blowup, n_cols, lde, lde_stride, layers_dev, s);
   if (e != cudaSuccess) return cuda_status(e, "commit_columns");
-  return read_root(root_host, layers_dev, log_size + log_blowup, s, "commit_columns root readback");
+  return read_root(ctx, root_host, layers_dev, log_size + log_blowup, s, "commit_columns root readback");
 }
 
 int32_t stwo_b200_interpolate_secure_composition(stwo_b200_context* ctx, uint32_t comp_log, uint32_t* comp,
@@ -409,8 +391,17 @@ int32_t stwo_b200_accumulate_quotients(stwo_b200_context* ctx, uint32_t log_size
   hb.sum_b = q(sum_b);
   hb.first = 0;
   hb.count = n_cols;
-  // The column pointers are read back so that 16-byte aligned columns may take the bulk-staged
-  // kernel, whose status word sits after the batch descriptor.
+  if (sb::tune_forced() < 3) {
+    // The batch travels as a launch argument and the kernel looks at the column pointers itself. The
+    // result is complete on return, as it is below.
+    cudaError_t e = sb::accumulate_quotients(ctx->ctx.tables, log_size, 1, n_cols, nullptr, col_ptrs_dev,
+                                             reinterpret_cast<const sb::QM31*>(c_dev), out, out_stride, st(stream),
+                                             nullptr, &hb);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st(stream));
+    return cuda_status(e, "accumulate_quotients");
+  }
+  // The bulk-staged kernel is forced: the column pointers are read back, since it takes 16-byte aligned
+  // columns only, and its status word sits after the batch descriptor.
   std::vector<const uint32_t*> hptr(n_cols);
   cudaError_t e = cudaMemcpyAsync(hptr.data(), col_ptrs_dev, n_cols * sizeof(void*), cudaMemcpyDeviceToHost, st(stream));
   if (e == cudaSuccess) e = cudaStreamSynchronize(st(stream));

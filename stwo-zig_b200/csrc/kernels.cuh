@@ -104,7 +104,8 @@ struct QuotientBatchDev {
   uint32_t first, count; // range in the column/coefficient lists
 };
 // Single-size quotient: all columns have log size `log_size` (the lifting size).
-// col_ptrs/coeff_c are device arrays of length n_entries; batches device array.
+// col_ptrs/coeff_c are device arrays of length n_entries; batches device array, or null with the single
+// batch in host memory at `one` (not with a status word).
 // `status` (device word, may be null): a caller that passes one vouches that every column pointer is
 // 16-byte aligned, which allows 16-byte copies of them and, as a forced variant, the bulk-staged kernel, which ORs
 // QUOT_STATUS_* bits into it when a staged load runs out of time or the batches do not fit its
@@ -113,7 +114,8 @@ constexpr uint32_t QUOT_STATUS_TIMEOUT = 2, QUOT_STATUS_LAYOUT = 4;
 cudaError_t accumulate_quotients(const DeviceTables& t, uint32_t log_size, uint32_t n_batches, uint32_t n_entries,
                                  const QuotientBatchDev* batches, const uint32_t* const* col_ptrs,
                                  const QM31* coeff_c, uint32_t* out, uint64_t out_stride,
-                                 cudaStream_t stream, uint32_t* status = nullptr);
+                                 cudaStream_t stream, uint32_t* status = nullptr,
+                                 const QuotientBatchDev* one = nullptr);
 // Test hook: the next bulk-staged quotient launch leaves its first stage empty in every CTA, so that
 // its bounded waits run out (status QUOT_STATUS_TIMEOUT).
 void arm_quotient_stage_timeout_for_testing();
@@ -130,10 +132,10 @@ cudaError_t fold_line(const DeviceTables& t, uint32_t src_log, const uint32_t* s
 // domain halfOdds(src_log)) fused with the commitment of the folded layer: when
 // `layers` is non-null the folded values are hashed as leaves (4 words each) and
 // the whole tree of 2^(src_log-1) leaves is built. `alpha` is device memory (written
-// by fri_channel_step earlier on the same stream).
+// by fri_channel_step earlier on the same stream), or null with the value in `alpha_v`.
 cudaError_t fri_fold_commit(const DeviceTables& t, bool circle, uint32_t src_log, const uint32_t* src,
                             uint64_t src_stride, const QM31* alpha, uint32_t* dst, uint64_t dst_stride,
-                            uint8_t* layers, cudaStream_t stream);
+                            uint8_t* layers, cudaStream_t stream, QM31 alpha_v = qzero());
 
 // Blake2s Fiat-Shamir channel state on the device for the FRI commit phase
 // (src/prover/fri.zig:314-592: per layer mixRoot, then drawSecureFelt for its alpha), so

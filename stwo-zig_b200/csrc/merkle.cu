@@ -443,7 +443,7 @@ __device__ __forceinline__ void fri_ibfly(QM31& f0, QM31& f1, uint32_t it) {
 template <bool CIRCLE>
 __global__ void __launch_bounds__(LEAF_THREADS) k_fri_fold_commit(TwiddleView itv, uint32_t dst_log,
                                                                    const uint32_t* __restrict__ src, uint64_t ss,
-                                                                   const QM31* alpha_p, uint32_t* dst, uint64_t ds,
+                                                                   const QM31* alpha_p, QM31 alpha_v, uint32_t* dst, uint64_t ds,
                                                                    uint8_t* layers, Seeds seeds, uint32_t levels,
                                                                    uint32_t one) {
   chain_enter();
@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(LEAF_THREADS) k_fri_fold_commit(TwiddleView it
   const uint64_t n = 1ull << dst_log;
   const uint64_t i = (uint64_t)blockIdx.x * LEAF_THREADS + threadIdx.x;
   if (i < n) {
-    const QM31 alpha = *alpha_p;
+    const QM31 alpha = alpha_p ? *alpha_p : alpha_v;
     uint2 w0 = *reinterpret_cast<const uint2*>(src + 2 * i);
     uint2 w1 = *reinterpret_cast<const uint2*>(src + ss + 2 * i);
     uint2 w2 = *reinterpret_cast<const uint2*>(src + 2 * ss + 2 * i);
@@ -744,7 +744,7 @@ cudaError_t fri_channel_step(FriChannelDev* c, const uint8_t* root, uint32_t slo
 
 cudaError_t fri_fold_commit(const DeviceTables& t, bool circle, uint32_t src_log, const uint32_t* src,
                             uint64_t src_stride, const QM31* alpha, uint32_t* dst, uint64_t dst_stride,
-                            uint8_t* layers, cudaStream_t stream) {
+                            uint8_t* layers, cudaStream_t stream, QM31 alpha_v) {
   const Seeds& seeds = seeds_once();
   const uint32_t dst_log = src_log - 1;
   const uint64_t n = 1ull << dst_log;
@@ -754,10 +754,10 @@ cudaError_t fri_fold_commit(const DeviceTables& t, bool circle, uint32_t src_log
   cudaError_t e;
   if (circle)
     e = launch_chained(k_fri_fold_commit<true>, grid, LEAF_THREADS, 0, stream, t.view(src_log, true), dst_log, src,
-                       src_stride, alpha, dst, dst_stride, layers, seeds, levels, 1u);
+                       src_stride, alpha, alpha_v, dst, dst_stride, layers, seeds, levels, 1u);
   else
     e = launch_chained(k_fri_fold_commit<false>, grid, LEAF_THREADS, 0, stream, t.view(src_log + 1, true), dst_log, src,
-                       src_stride, alpha, dst, dst_stride, layers, seeds, levels, 1u);
+                       src_stride, alpha, alpha_v, dst, dst_stride, layers, seeds, levels, 1u);
   note_launch();
   if (e != cudaSuccess || !layers) return e;
   return merkle_finish(layers, dst_log, dst_log - levels, stream);

@@ -100,6 +100,31 @@ size_t layout_bytes(const Layout& l) {
 // ---------------------------------------------------------------------------
 // Context
 // ---------------------------------------------------------------------------
+PinnedSlots::~PinnedSlots() {
+  if (base_) cudaFreeHost(base_);
+}
+void PinnedSlots::init() {
+  if (cudaMallocHost(reinterpret_cast<void**>(&base_), COUNT * BYTES) != cudaSuccess) {
+    cudaGetLastError();
+    base_ = nullptr;
+    return;
+  }
+  free_.store(~0u);
+}
+PinnedSlots::Slot::Slot(PinnedSlots& p) : pool_(p) {
+  uint32_t f = p.free_.load();
+  while (f) {
+    const uint32_t i = (uint32_t)__builtin_ctz(f);
+    if (p.free_.compare_exchange_weak(f, f & ~(1u << i))) {
+      index_ = i;
+      return;
+    }
+  }
+}
+PinnedSlots::Slot::~Slot() {
+  if (index_ < COUNT) pool_.free_.fetch_or(1u << index_);
+}
+
 Context::~Context() {
   for (WideFibProver* p : pool) delete p;
   for (LogupXorProver* p : xor_pool) delete p;
@@ -126,6 +151,7 @@ int32_t Context::init(int dev, uint32_t tower_log) {
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &threshold);
   }
   if (cudaMalloc(&small, 256) != cudaSuccess) return E_OOM;
+  slots.init();
   std::vector<PointM> pts = build_point_table();
   if (cudaMalloc(&tables.points, pts.size() * sizeof(PointM)) != cudaSuccess) return E_OOM;
   if (cudaMemcpy(tables.points, pts.data(), pts.size() * sizeof(PointM), cudaMemcpyHostToDevice) != cudaSuccess)

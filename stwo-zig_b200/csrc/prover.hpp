@@ -4,6 +4,7 @@
 
 #include <chrono>
 #include <cstdint>
+#include <atomic>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -165,8 +166,38 @@ class LogupXorProver {
   Deadline deadline_;
 };
 
+// A fixed number of small page-locked buffers for results that the op-level calls read back (a copy into
+// pageable memory is staged by the runtime). A call holds one while its copy is in flight; when all are
+// taken, or the allocation failed, data() is null and the call copies into the caller's memory directly.
+class PinnedSlots {
+ public:
+  static constexpr uint32_t COUNT = 32, BYTES = 64;
+  PinnedSlots() = default;
+  PinnedSlots(const PinnedSlots&) = delete;
+  PinnedSlots& operator=(const PinnedSlots&) = delete;
+  ~PinnedSlots();
+  void init();
+  class Slot {
+   public:
+    explicit Slot(PinnedSlots& p);
+    ~Slot();
+    Slot(const Slot&) = delete;
+    Slot& operator=(const Slot&) = delete;
+    uint8_t* data() const { return index_ < COUNT ? pool_.base_ + index_ * BYTES : nullptr; }
+
+   private:
+    PinnedSlots& pool_;
+    uint32_t index_ = COUNT;
+  };
+
+ private:
+  uint8_t* base_ = nullptr;
+  std::atomic<uint32_t> free_{0};  // bit i: slot i is free
+};
+
 struct Context {
   int device = 0;
+  PinnedSlots slots;
   int sm_count = 0;
   DeviceTables tables;
   std::mutex mu;

@@ -451,10 +451,12 @@ __global__ void k_oods_sum(const QM31* partial, uint32_t n_chunks, uint32_t n_co
 constexpr uint32_t QUOT_MAX_ENTRIES = 1024;
 
 __global__ void __launch_bounds__(256) k_quotients(PointTable pts, uint32_t log_size, uint32_t n_batches,
-                                                   const QuotientBatchDev* __restrict__ batches,
+                                                   const QuotientBatchDev* batches,
+                                                   const __grid_constant__ QuotientBatchDev one,
                                                    const uint32_t* const* __restrict__ col_ptrs,
                                                    const QM31* __restrict__ coeff_c, uint32_t* out, uint64_t out_stride) {
   extern __shared__ uint32_t sq[];  // 4 words per entry
+  if (!batches) batches = &one;
   uint32_t n_entries = 0;
   for (uint32_t b = 0; b < n_batches; ++b) n_entries = max(n_entries, batches[b].first + batches[b].count);
   for (uint32_t i = threadIdx.x; i < n_entries; i += blockDim.x) qstore4(coeff_c[i], sq + 4 * i);
@@ -530,25 +532,10 @@ __device__ __forceinline__ void quot_batch_finish(const QuotientBatchDev& bt, co
 // Bound by HBM: 2^21 rows x 108 columns 168 us, 5.6 TB/s (the lazily accumulating register
 // kernel, ten instructions per word, 265 us; the bulk-staged one 258 us).
 template <bool ALIGNED>
-__global__ void __launch_bounds__(MMA_THREADS, 3) k_quotients_mma(PointTable pts, uint32_t log_size, uint32_t n_batches,
-                                                                  const QuotientBatchDev* __restrict__ batches,
-                                                                  const uint32_t* const* __restrict__ col_ptrs,
-                                                                  const QM31* __restrict__ coeff_c, uint32_t padded,
-                                                                  uint32_t* out, uint64_t out_stride) {
-  extern __shared__ uint4 qmma[];
-  uint32_t* sq = reinterpret_cast<uint32_t*>(qmma + mma_ring_bytes(QUOT_STAGES) / 16);  // byte-reversed coefficients
-  const uint32_t** sptr = reinterpret_cast<const uint32_t**>(sq + 4 * padded);  // column pointers
-  uint32_t total = 0;  // steps of eight entries of all batches
-  for (uint32_t b = 0; b < n_batches; ++b) {
-    const uint32_t first = batches[b].first, count = batches[b].count, room = (count + 7) / 8 * 8;
-    for (uint32_t i = threadIdx.x; i < room; i += MMA_THREADS) {
-      const uint32_t e = first + (i < count ? i : 0);
-      put_reversed(sq + 4 * (8 * total + i), i < count ? coeff_c[e] : qzero());
-      sptr[8 * total + i] = col_ptrs[e];
-    }
-    total += room / 8;
-  }
-  __syncthreads();
+__device__ __forceinline__ void quotients_mma_rows(const PointTable& pts, uint32_t log_size, uint32_t n_batches,
+                                                   const QuotientBatchDev* batches, uint4* qmma, const uint32_t* sq,
+                                                   const uint32_t* const* sptr, uint32_t total, uint32_t* out,
+                                                   uint64_t out_stride) {
   const uint32_t lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const mmadot::LaneShifts shifts = mmadot::lane_shifts(g & 1);
   const uint32_t n_blocks = (1u << log_size) / MMA_ROWS, warps = gridDim.x * (MMA_THREADS / 32);
@@ -622,6 +609,41 @@ __global__ void __launch_bounds__(MMA_THREADS, 3) k_quotients_mma(PointTable pts
     for (int m = 0; m < 4; ++m)
       store_rows2<ALIGNED>(out + t * out_stride + row0 + 16 * m, make_uint2(num[m][0], num[m][1]));
   }
+}
+
+// batches == nullptr: the one batch `one`. CHECK: the kernel looks at the column pointers itself (a caller that
+// vouches for their alignment takes the other).
+template <bool CHECK>
+__global__ void __launch_bounds__(MMA_THREADS, 3) k_quotients_mma(PointTable pts, uint32_t log_size, uint32_t n_batches,
+                                                                  const QuotientBatchDev* batches,
+                                                                  const __grid_constant__ QuotientBatchDev one,
+                                                                  const uint32_t* const* __restrict__ col_ptrs,
+                                                                  const QM31* __restrict__ coeff_c, uint32_t padded,
+                                                                  uint32_t* out, uint64_t out_stride) {
+  extern __shared__ uint4 qmma[];
+  __shared__ int s_bad;
+  if (!batches) batches = &one;
+  uint32_t* sq = reinterpret_cast<uint32_t*>(qmma + mma_ring_bytes(QUOT_STAGES) / 16);  // byte-reversed coefficients
+  const uint32_t** sptr = reinterpret_cast<const uint32_t**>(sq + 4 * padded);  // column pointers
+  if (CHECK) {
+    if (threadIdx.x == 0) s_bad = (reinterpret_cast<uintptr_t>(out) & 15) != 0 || out_stride % 4 != 0;
+    __syncthreads();
+  }
+  uint32_t total = 0;  // steps of eight entries of all batches
+  for (uint32_t b = 0; b < n_batches; ++b) {
+    const uint32_t first = batches[b].first, count = batches[b].count, room = (count + 7) / 8 * 8;
+    for (uint32_t i = threadIdx.x; i < room; i += MMA_THREADS) {
+      const uint32_t e = first + (i < count ? i : 0);
+      put_reversed(sq + 4 * (8 * total + i), i < count ? coeff_c[e] : qzero());
+      const uint32_t* p = col_ptrs[e];
+      sptr[8 * total + i] = p;
+      if (CHECK && (reinterpret_cast<uintptr_t>(p) & 15)) s_bad = 1;
+    }
+    total += room / 8;
+  }
+  __syncthreads();
+  if (CHECK && s_bad) quotients_mma_rows<false>(pts, log_size, n_batches, batches, qmma, sq, sptr, total, out, out_stride);
+  else quotients_mma_rows<true>(pts, log_size, n_batches, batches, qmma, sq, sptr, total, out, out_stride);
 }
 
 // ---- Quotients with the column words staged in shared memory by bulk async copies ----------
@@ -1041,7 +1063,8 @@ void arm_quotient_stage_timeout_for_testing() { g_quot_skip_first_item.store(tru
 
 cudaError_t accumulate_quotients(const DeviceTables& t, uint32_t log_size, uint32_t n_batches, uint32_t n_entries,
                                  const QuotientBatchDev* batches, const uint32_t* const* col_ptrs, const QM31* coeff_c,
-                                 uint32_t* out, uint64_t out_stride, cudaStream_t stream, uint32_t* status) {
+                                 uint32_t* out, uint64_t out_stride, cudaStream_t stream, uint32_t* status,
+                                 const QuotientBatchDev* one) {
   const size_t smem = QUOT_MAX_ENTRIES * 16;
   // Tensor-core kernel: every batch padded to a multiple of eight entries.
   const uint32_t padded = n_entries + 7 * n_batches;
@@ -1066,8 +1089,9 @@ cudaError_t accumulate_quotients(const DeviceTables& t, uint32_t log_size, uint3
   (void)attr;
   // The tensor-core kernel takes whole blocks of 64 rows.
   if ((1ull << log_size) < MMA_ROWS || smem_m > SMEM_M_MAX) {
-    k_quotients<<<grid_for(1ull << log_size, 256), 256, smem, stream>>>(PointTable{t.points}, log_size, n_batches,
-                                                                        batches, col_ptrs, coeff_c, out, out_stride);
+    k_quotients<<<grid_for(1ull << log_size, 256), 256, smem, stream>>>(PointTable{t.points}, log_size, n_batches, batches,
+                                                                        one ? *one : QuotientBatchDev{}, col_ptrs,
+                                                                        coeff_c, out, out_stride);
     note_launch();
     return cudaGetLastError();
   }
@@ -1091,12 +1115,12 @@ cudaError_t accumulate_quotients(const DeviceTables& t, uint32_t log_size, uint3
                                                         item_cap, out, out_stride, status, skip);
     } else {
       // Persistent: three CTAs per SM, each warp 64 rows at a time. Sixteen-byte copies where the caller
-      // vouches for the columns and the output allows them.
+      // vouches for the columns and the output allows them, or the kernel finds them aligned.
       const uint32_t blocks = (uint32_t)((1ull << log_size) / MMA_ROWS), per_cta = MMA_THREADS / 32;
       const uint32_t g = std::min<uint32_t>((blocks + per_cta - 1) / per_cta, t.sm_count * 3);
       const bool aligned = status != nullptr && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && out_stride % 4 == 0;
-      (aligned ? k_quotients_mma<true> : k_quotients_mma<false>)<<<g, MMA_THREADS, smem_m, stream>>>(
-          pts, log_size, n_batches, batches, col_ptrs, coeff_c, padded, out, out_stride);
+      (aligned ? k_quotients_mma<false> : k_quotients_mma<true>)<<<g, MMA_THREADS, smem_m, stream>>>(
+          pts, log_size, n_batches, batches, one ? *one : QuotientBatchDev{}, col_ptrs, coeff_c, padded, out, out_stride);
     }
     note_launch();
     return cudaGetLastError();

@@ -80,6 +80,8 @@ cudaError_t tuned_run(TuneOp op, uint32_t log_size, uint32_t n_cols, int n_varia
 
 void tune_force(int v) { g_force.store(v < 0 ? -1 : v, std::memory_order_relaxed); }
 
+int tune_forced() { return g_force.load(std::memory_order_relaxed); }
+
 std::vector<TuneEntry> tune_table() {
   Table& t = table();
   std::lock_guard<std::mutex> g(t.mu);

@@ -34,6 +34,7 @@ cudaError_t tuned_run(TuneOp op, uint32_t log_size, uint32_t n_cols, int n_varia
                       cudaStream_t stream, const std::function<cudaError_t(int)>& run);
 // -1: tune (the default); v >= 0: every op runs variant min(v, its count - 1) and nothing is tuned.
 void tune_force(int v);
+int tune_forced();  // the forced variant, or -1
 std::vector<TuneEntry> tune_table();
 void tune_clear();
 
