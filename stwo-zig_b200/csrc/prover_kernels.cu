@@ -136,8 +136,8 @@ constexpr int MMA_THREADS = 128;
 // A read-only probe of this walk (108 columns of 2^21 rows) runs at 6.9 TB/s; with each lane copying its
 // own operand words (neighbour lanes on four different columns) it stays at 3.9 TB/s at any depth, and
 // with the same depth in registers the quotients took 325 us.
-// Stages of the composition (four CTAs per SM: 124 registers) and of the quotients (three: 168).
-constexpr int COMP_STAGES = 4, QUOT_STAGES = 6;
+// Stages of the composition and of the quotients (four CTAs per SM each).
+constexpr int COMP_STAGES = 4, QUOT_STAGES = 5;
 constexpr uint32_t MMA_ROWS = 64;           // rows of a warp's block
 constexpr uint32_t MMA_COL = 4 * MMA_ROWS + 32;   // bytes between a stage's columns
 constexpr uint32_t MMA_STAGE = 8 * MMA_COL;       // bytes of a warp's stage
@@ -569,6 +569,11 @@ __device__ __forceinline__ void quotients_mma_rows(const PointTable& pts, uint32
         acc.step(w, q[0], q[16], shifts);
         fetch();
       }
+      uint32_t sum[4][2];  // before the denominators: it ends the accumulators' registers
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int s = 0; s < 2; ++s) sum[m][s] = mmadot::row_sum(acc, m, s);
       const PointM at = padd(plo, phi);
       CM31 inv[2];
       {
@@ -597,7 +602,7 @@ __device__ __forceinline__ void quotients_mma_rows(const PointTable& pts, uint32
         for (int s = 0; s < 2; ++s) {
           const CM31 iv = {__shfl_sync(0xffffffffu, inv[s].a, m, 4), __shfl_sync(0xffffffffu, inv[s].b, m, 4)};
           const uint32_t line = s ? msub(sum_b, ay) : madd(sum_b, ay);
-          const uint32_t v = msub(mmadot::row_sum(acc, m, s), line);
+          const uint32_t v = msub(sum[m][s], line);
           // (v0 + v1 i)(a + b i): lane t holds v0 (even) or v1 (odd) of its half and keeps that coordinate.
           const uint32_t o = __shfl_xor_sync(0xffffffffu, v, 1);
           const uint32_t va = mmul(v, iv.a), ob = mmul(o, iv.b);
@@ -614,7 +619,7 @@ __device__ __forceinline__ void quotients_mma_rows(const PointTable& pts, uint32
 // batches == nullptr: the one batch `one`. CHECK: the kernel looks at the column pointers itself (a caller that
 // vouches for their alignment takes the other).
 template <bool CHECK>
-__global__ void __launch_bounds__(MMA_THREADS, 3) k_quotients_mma(PointTable pts, uint32_t log_size, uint32_t n_batches,
+__global__ void __launch_bounds__(MMA_THREADS, 4) k_quotients_mma(PointTable pts, uint32_t log_size, uint32_t n_batches,
                                                                   const QuotientBatchDev* batches,
                                                                   const __grid_constant__ QuotientBatchDev one,
                                                                   const uint32_t* const* __restrict__ col_ptrs,
@@ -1114,10 +1119,10 @@ cudaError_t accumulate_quotients(const DeviceTables& t, uint32_t log_size, uint3
         k_quotients_bulk<2><<<g, QB_THREADS, smem_b, stream>>>(pts, log_size, n_batches, batches, col_ptrs, coeff_c, n_entries,
                                                         item_cap, out, out_stride, status, skip);
     } else {
-      // Persistent: three CTAs per SM, each warp 64 rows at a time. Sixteen-byte copies where the caller
+      // Persistent: four CTAs per SM, each warp 64 rows at a time. Sixteen-byte copies where the caller
       // vouches for the columns and the output allows them, or the kernel finds them aligned.
       const uint32_t blocks = (uint32_t)((1ull << log_size) / MMA_ROWS), per_cta = MMA_THREADS / 32;
-      const uint32_t g = std::min<uint32_t>((blocks + per_cta - 1) / per_cta, t.sm_count * 3);
+      const uint32_t g = std::min<uint32_t>((blocks + per_cta - 1) / per_cta, t.sm_count * 4);
       const bool aligned = status != nullptr && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && out_stride % 4 == 0;
       (aligned ? k_quotients_mma<false> : k_quotients_mma<true>)<<<g, MMA_THREADS, smem_m, stream>>>(
           pts, log_size, n_batches, batches, one ? *one : QuotientBatchDev{}, col_ptrs, coeff_c, padded, out, out_stride);
