@@ -151,3 +151,20 @@ def test_xor_lookup_interaction(ctx, log_n):
         assert np.array_equal(_host(inter_main).reshape(1, 4, rows), ref_m)
         assert np.array_equal(_host(inter_table).reshape(1, 4, 65536), ref_t)
         assert root == oracle.merkle_root([*ref_m[0], *ref_t[0]])
+
+
+@pytest.mark.parametrize("n_uses,batch,n_words", [(1, 1, 8), (2, 1, 3), (4, 1, 4), (4, 2, 7), (7, 2, 6), (9, 2, 2)])
+def test_fractions_by_column_count(ctx, n_uses, batch, n_words):
+    """One to four columns keep a row's fractions in registers, five take the general kernel; up to eight words
+    a use, the largest words among them."""
+    rng = np.random.default_rng(10 * n_uses + n_words)
+    rows = 1 << 9
+    cols = [rng.integers(0, P, size=rows, dtype=np.uint32) for _ in range(n_words)]
+    for c in cols:
+        c[:4] = P - 1
+    mult = rng.integers(0, P, size=rows, dtype=np.uint32)
+    uses = [dict(words=[cols[(u + j) % n_words] for j in range(n_words)], multiplicity=mult if u % 2 else None,
+                 negate=u % 3 == 1) for u in range(n_uses)]
+    alphas = [rng.integers(0, P, size=4).tolist() for _ in range(n_words)]
+    ref, rc, got, gc = _run_both(ctx, 9, uses, alphas, rng.integers(0, P, size=4).tolist(), batch, 1)
+    assert np.array_equal(got, ref) and np.array_equal(gc, rc)
