@@ -152,29 +152,33 @@ __device__ __forceinline__ QM31 shfl_up_q(QM31 v, int d) {
                __shfl_up_sync(0xffffffffu, v.c1.a, d), __shfl_up_sync(0xffffffffu, v.c1.b, d));
 }
 
-// Inclusive scan of one QM31 per thread over a CTA of LU_THREADS threads; also returns the CTA total.
-__device__ __forceinline__ QM31 block_inclusive_scan(QM31 v, QM31& total) {
-  __shared__ QM31 warp_sums[LU_THREADS / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// Inclusive scan over a warp.
+__device__ __forceinline__ QM31 warp_inclusive_scan(QM31 v) {
+  const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
-    QM31 o = shfl_up_q(v, d);
+    const QM31 o = shfl_up_q(v, d);
     if (lane >= d) v = qadd(v, o);
   }
+  return v;
+}
+
+// Inclusive scan of one QM31 per thread over a CTA of THREADS threads; also returns the CTA total.
+template <int THREADS>
+__device__ __forceinline__ QM31 block_inclusive_scan(QM31 v, QM31& total) {
+  constexpr int WARPS = THREADS / 32;
+  __shared__ QM31 warp_sums[WARPS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  v = warp_inclusive_scan(v);
   if (lane == 31) warp_sums[warp] = v;
   __syncthreads();
   if (warp == 0) {
-    QM31 w = lane < LU_THREADS / 32 ? warp_sums[lane] : qzero();
-#pragma unroll
-    for (int d = 1; d < LU_THREADS / 32; d <<= 1) {
-      QM31 o = shfl_up_q(w, d);
-      if (lane >= d) w = qadd(w, o);
-    }
-    if (lane < LU_THREADS / 32) warp_sums[lane] = w;
+    const QM31 w = warp_inclusive_scan(lane < WARPS ? warp_sums[lane] : qzero());
+    if (lane < WARPS) warp_sums[lane] = w;
   }
   __syncthreads();
   if (warp > 0) v = qadd(v, warp_sums[warp - 1]);
-  total = warp_sums[LU_THREADS / 32 - 1];
+  total = warp_sums[WARPS - 1];
   return v;
 }
 
@@ -187,28 +191,28 @@ __global__ void __launch_bounds__(LU_THREADS) k_logup_block_sums(const uint32_t*
   for (int k = 0; k < SCAN_PER_THREAD; ++k)
     if (s0 + k < rows) sum = qadd(sum, col_load(col, stride, 0, scan_row(s0 + k, log_rows, order)));
   QM31 total;
-  block_inclusive_scan(sum, total);
+  block_inclusive_scan<LU_THREADS>(sum, total);
   if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
 }
 
-// One CTA: block_sums[b] <- sum of blocks before b; *claimed <- sum of all.
-__global__ void __launch_bounds__(LU_THREADS) k_logup_scan_blocks(QM31* block_sums, uint32_t n_blocks,
-                                                                  QM31* claimed) {
-  const uint32_t per = (n_blocks + LU_THREADS - 1) / LU_THREADS;
-  const uint32_t b0 = threadIdx.x * per;
-  QM31 sum = qzero();
-  for (uint32_t i = 0; i < per; ++i)
-    if (b0 + i < n_blocks) sum = qadd(sum, block_sums[b0 + i]);
-  QM31 total;
-  QM31 incl = block_inclusive_scan(sum, total);
-  QM31 run = qsub(incl, sum);  // exclusive prefix of this thread's chunk
-  for (uint32_t i = 0; i < per; ++i) {
-    if (b0 + i >= n_blocks) break;
-    QM31 v = block_sums[b0 + i];
-    block_sums[b0 + i] = run;
-    run = qadd(run, v);
+// One CTA: block_sums[b] <- sum of blocks before b; *claimed <- sum of all. 1024 sums at a time, contiguous
+// across the threads, the next ones fetched while these are scanned (each thread summing a run of its own
+// took 55 us for 8192 sums).
+constexpr int SCAN_THREADS = 1024;
+__global__ void __launch_bounds__(SCAN_THREADS) k_logup_scan_blocks(QM31* block_sums, uint32_t n_blocks,
+                                                                    QM31* claimed) {
+  QM31 carry = qzero();
+  QM31 v = threadIdx.x < n_blocks ? block_sums[threadIdx.x] : qzero();
+  for (uint32_t b = threadIdx.x, base = 0; base < n_blocks; base += SCAN_THREADS, b += SCAN_THREADS) {
+    const QM31 next = (uint64_t)b + SCAN_THREADS < n_blocks ? block_sums[b + SCAN_THREADS] : qzero();
+    QM31 total;
+    const QM31 incl = block_inclusive_scan<SCAN_THREADS>(v, total);
+    if (b < n_blocks) block_sums[b] = qadd(carry, qsub(incl, v));
+    carry = qadd(carry, total);
+    v = next;
+    __syncthreads();  // the scan's shared words are written again
   }
-  if (threadIdx.x == 0) *claimed = total;
+  if (threadIdx.x == 0) *claimed = carry;
 }
 
 __global__ void __launch_bounds__(LU_THREADS) k_logup_finalize(uint32_t* col, uint64_t stride, uint32_t log_rows,
@@ -224,7 +228,7 @@ __global__ void __launch_bounds__(LU_THREADS) k_logup_finalize(uint32_t* col, ui
     sum = qadd(sum, v[k]);
   }
   QM31 total_block;
-  QM31 incl = block_inclusive_scan(sum, total_block);
+  QM31 incl = block_inclusive_scan<LU_THREADS>(sum, total_block);
   QM31 run = qadd(block_prefix[blockIdx.x], qsub(incl, sum));
   const QM31 total = *claimed;
   // 1/N = 2^(31 - log_rows) in M31 (2^31 = 1).
@@ -238,6 +242,97 @@ __global__ void __launch_bounds__(LU_THREADS) k_logup_finalize(uint32_t* col, ui
     if (order == 1) out = qsub(out, qmulm(total, mmul(inv_rows, (uint32_t)((s + 1) % P))));
     col_store(col, stride, 0, scan_row(s, log_rows, order), out);
   }
+}
+
+// ---- The coset-order scan by whole memory sectors (2^10 rows or more, 16-byte aligned columns) ------------------
+// Coset positions 2j and 2j + 1 (j < N / 2) are rows r = 2 bitrev(j) and N - 1 - r, so consecutive positions lie
+// a large power of two apart and a row-by-row gather fetches a 32-byte sector for every word (2^20 rows: 20 us for
+// the block sums, 58 us for the final pass). With j = (a, m, l), a its top two bits and l its lowest six, the
+// sector of eight rows at (bitrev l, bitrev m, 000) holds the even positions of (a, m, l) for the four a and, by
+// the complement, the odd ones of (a, ~m, ~l): a CTA that takes m and ~m with every a and l reads 128 whole
+// sectors of each coordinate and owns eight segments of 128 consecutive positions, one per warp. The segments'
+// sums are scanned as the blocks' are. Now 7.7 and 12.8 us.
+constexpr uint32_t SEG = 128;           // positions of a segment
+constexpr uint32_t COSET_MIN_LOG = 10;  // at least one bit of m
+
+struct CosetTile {
+  uint32_t log, mid_bits, m;  // log rows, bits of m, this CTA's m (its complement is the other one)
+  __device__ __forceinline__ explicit CosetTile(uint32_t log_rows) : log(log_rows), mid_bits(log_rows - 9), m(blockIdx.x) {}
+  // First row of this thread's four (half a sector).
+  __device__ __forceinline__ uint64_t row() const {
+    const uint32_t q = threadIdx.x >> 1, l = q & 63;
+    return ((uint64_t)(__brev(l) >> 26) << (log - 6)) | ((uint64_t)(__brev(mid(q >> 6)) >> (32 - mid_bits)) << 3) |
+           (4 * (threadIdx.x & 1));
+  }
+  __device__ __forceinline__ uint32_t mid(uint32_t sel) const { return sel ? (1u << mid_bits) - 1 - m : m; }
+  // Place (segment * SEG + position in it) of the thread's i-th word.
+  __device__ __forceinline__ static uint32_t place(int i) {
+    const uint32_t q = threadIdx.x >> 1, l = q & 63, sel = q >> 6, w = 4 * (threadIdx.x & 1) + i;
+    const uint32_t k = (w & 1 ? 7 - w : w) >> 1, a = ((k & 1) << 1) | (k >> 1);
+    return w & 1 ? ((1 - sel) * 4 + a) * SEG + 2 * (63 - l) + 1 : (sel * 4 + a) * SEG + 2 * l;
+  }
+  // Number of segment `seg` (0..7) of this CTA among all of the scan's.
+  __device__ __forceinline__ uint32_t segment(uint32_t seg) const { return ((seg & 3) << mid_bits) | mid(seg >> 2); }
+};
+
+// The CTA's rows, by coordinate and place.
+__device__ __forceinline__ void coset_load(const CosetTile& t, const uint32_t* col, uint64_t stride, uint32_t (&v)[4][8 * SEG]) {
+  const uint64_t row = t.row();
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const uint4 x = *reinterpret_cast<const uint4*>(col + c * stride + row);
+    v[c][t.place(0)] = x.x; v[c][t.place(1)] = x.y; v[c][t.place(2)] = x.z; v[c][t.place(3)] = x.w;
+  }
+  __syncthreads();
+}
+// Lane's four consecutive positions of its warp's segment.
+__device__ __forceinline__ void coset_lane(const uint32_t (&v)[4][8 * SEG], QM31 (&x)[4]) {
+  const uint32_t at = threadIdx.x * 4;
+  uint4 c[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) c[k] = *reinterpret_cast<const uint4*>(&v[k][at]);
+  x[0] = qmake(c[0].x, c[1].x, c[2].x, c[3].x);
+  x[1] = qmake(c[0].y, c[1].y, c[2].y, c[3].y);
+  x[2] = qmake(c[0].z, c[1].z, c[2].z, c[3].z);
+  x[3] = qmake(c[0].w, c[1].w, c[2].w, c[3].w);
+}
+
+__global__ void __launch_bounds__(LU_THREADS) k_logup_coset_sums(const uint32_t* col, uint64_t stride, uint32_t log_rows,
+                                                                 QM31* seg_sums) {
+  __shared__ __align__(16) uint32_t v[4][8 * SEG];
+  const CosetTile t(log_rows);
+  coset_load(t, col, stride, v);
+  QM31 x[4];
+  coset_lane(v, x);
+  const QM31 incl = warp_inclusive_scan(qadd(qadd(x[0], x[1]), qadd(x[2], x[3])));
+  if ((threadIdx.x & 31) == 31) seg_sums[t.segment(threadIdx.x >> 5)] = incl;
+}
+
+__global__ void __launch_bounds__(LU_THREADS) k_logup_coset_finalize(uint32_t* col, uint64_t stride, uint32_t log_rows,
+                                                                     const QM31* seg_prefix, const QM31* claimed) {
+  __shared__ __align__(16) uint32_t v[4][8 * SEG];
+  const CosetTile t(log_rows);
+  coset_load(t, col, stride, v);
+  QM31 x[4];
+  coset_lane(v, x);
+  const QM31 sum = qadd(qadd(x[0], x[1]), qadd(x[2], x[3]));
+  const uint32_t seg = t.segment(threadIdx.x >> 5);
+  QM31 run = qadd(seg_prefix[seg], qsub(warp_inclusive_scan(sum), sum));
+  const QM31 step = qmulm(*claimed, 1u << (31 - log_rows));  // total / N: 1 / N = 2^(31 - log_rows) in M31
+  const uint64_t s0 = (uint64_t)seg * SEG + 4 * (threadIdx.x & 31);
+  const uint32_t at = threadIdx.x * 4;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    run = qadd(run, x[k]);
+    const QM31 o = qsub(run, qmulm(step, (uint32_t)((s0 + k + 1) % P)));
+    v[0][at + k] = o.c0.a; v[1][at + k] = o.c0.b; v[2][at + k] = o.c1.a; v[3][at + k] = o.c1.b;
+  }
+  __syncthreads();
+  const uint64_t row = t.row();
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    *reinterpret_cast<uint4*>(col + c * stride + row) =
+        make_uint4(v[c][t.place(0)], v[c][t.place(1)], v[c][t.place(2)], v[c][t.place(3)]);
 }
 
 uint32_t scan_blocks(uint32_t log_rows) {
@@ -279,7 +374,9 @@ __global__ void k_xor_table(uint32_t* table) {
 
 }  // namespace
 
-size_t logup_scratch_count(uint32_t log_rows) { return scan_blocks(log_rows); }
+size_t logup_scratch_count(uint32_t log_rows) {
+  return log_rows >= COSET_MIN_LOG ? (1ull << log_rows) / SEG : scan_blocks(log_rows);
+}
 
 cudaError_t logup_interaction(const LogupParams& p, uint32_t* out, uint64_t out_stride, QM31* claimed,
                               QM31* scratch, uint32_t* zero_flag, cudaStream_t stream) {
@@ -294,12 +391,17 @@ cudaError_t logup_interaction(const LogupParams& p, uint32_t* out, uint64_t out_
   fractions<<<(unsigned)((rows + LU_THREADS - 1) / LU_THREADS), LU_THREADS, 0, stream>>>(p, out, out_stride, zero_flag);
   note_launch();
   uint32_t* last = out + 4ull * (n_cols - 1) * out_stride;
-  const uint32_t nb = scan_blocks(p.log_rows);
-  k_logup_block_sums<<<nb, LU_THREADS, 0, stream>>>(last, out_stride, p.log_rows, p.order, scratch);
+  const bool sectors = p.order == 1 && p.log_rows >= COSET_MIN_LOG && (reinterpret_cast<uintptr_t>(last) & 15) == 0 &&
+                       out_stride % 4 == 0;
+  const uint32_t nb = sectors ? (uint32_t)(rows / SEG) : scan_blocks(p.log_rows);
+  if (sectors) k_logup_coset_sums<<<(unsigned)(rows / (8 * SEG)), LU_THREADS, 0, stream>>>(last, out_stride, p.log_rows, scratch);
+  else k_logup_block_sums<<<nb, LU_THREADS, 0, stream>>>(last, out_stride, p.log_rows, p.order, scratch);
   note_launch();
-  k_logup_scan_blocks<<<1, LU_THREADS, 0, stream>>>(scratch, nb, claimed);
+  k_logup_scan_blocks<<<1, SCAN_THREADS, 0, stream>>>(scratch, nb, claimed);
   note_launch();
-  k_logup_finalize<<<nb, LU_THREADS, 0, stream>>>(last, out_stride, p.log_rows, p.order, scratch, claimed);
+  if (sectors)
+    k_logup_coset_finalize<<<(unsigned)(rows / (8 * SEG)), LU_THREADS, 0, stream>>>(last, out_stride, p.log_rows, scratch, claimed);
+  else k_logup_finalize<<<nb, LU_THREADS, 0, stream>>>(last, out_stride, p.log_rows, p.order, scratch, claimed);
   note_launch();
   return cudaGetLastError();
 }

@@ -168,3 +168,16 @@ def test_fractions_by_column_count(ctx, n_uses, batch, n_words):
     alphas = [rng.integers(0, P, size=4).tolist() for _ in range(n_words)]
     ref, rc, got, gc = _run_both(ctx, 9, uses, alphas, rng.integers(0, P, size=4).tolist(), batch, 1)
     assert np.array_equal(got, ref) and np.array_equal(gc, rc)
+
+
+@pytest.mark.parametrize("log_rows,offset", [(10, 0), (10, 1), (11, 2), (12, 1)])
+def test_coset_scan_alignment(ctx, log_rows, offset):
+    """The scan by whole sectors takes 16-byte aligned columns from 2^10 rows; others go row by row."""
+    import torch
+    rng = np.random.default_rng(log_rows + offset)
+    col = rng.integers(0, P, size=1 << log_rows, dtype=np.uint32)
+    alphas, z = [rng.integers(0, P, size=4).tolist()], rng.integers(0, P, size=4).tolist()
+    ref, rc = oracle.logup_interaction(log_rows, [dict(words=[col])], alphas, z, batch=1, order=1)
+    out = torch.zeros((4 << log_rows) + offset, dtype=torch.int32, device="cuda")[offset:]
+    claimed = ctx.logup_interaction(log_rows, [dict(words=[_dev(col)])], alphas, z, out)
+    assert np.array_equal(_host(out).reshape(ref.shape), ref) and np.array_equal(np.array(claimed, dtype=np.uint32), rc)
