@@ -810,9 +810,9 @@ POW_INSTR_PER_NONCE = 943
 # XORs and rotations; the additions run on the FMA pipe.
 POW_ALU_INSTR_PER_NONCE = 567
 # Warp instructions of one interpolate + blow-up extend of a 2^20 column (ncu smsp__inst_executed.sum
-# of k_fft_low12<1, 0> + k_fft_high16_lde1<8> + k_fft_low12<0, 1>: 203.2 M + 391.0 M + 411.7 M for 100
+# of k_fft_low12<1, 0> + k_fft_high16_lde1<8> + k_fft_low12<0, 1>: 181.9 M + 361.7 M + 391.6 M for 100
 # columns).
-FFT_WARP_INSTR_PER_COL_2P20 = 1_005_824_000 // 100
+FFT_WARP_INSTR_PER_COL_2P20 = 935_168_000 // 100
 
 if __name__ == "__main__":
     main()
