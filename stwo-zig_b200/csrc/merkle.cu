@@ -583,14 +583,18 @@ __global__ void __launch_bounds__(QUAD_THREADS) k_fri_tail(FriChannelDev* c, con
   QuadLane L;
   quad_lane_init(L);
   cg::cluster_group cluster = cg::this_cluster();
-  cluster.barrier_arrive();  // every CTA runs before another one writes into its shared memory
   const uint32_t t = threadIdx.x, rank = blockIdx.x;
   uint32_t ctas = cluster.num_blocks(), log_ctas = __ffs(ctas) - 1;
   chain_enter();
-  if (t < 8) digest[t] = c->digest[t];
-  uint32_t root_word = 0;  // word t of the layer's root in threads 0..7
-  if (t < 8) root_word = reinterpret_cast<const uint32_t*>(p.tree[p.k0] + (2ull * (1u << (p.L - 1 - p.k0)) - 2) * 32)[t];
-  cluster.barrier_wait();
+  // The channel's state and, in threads 0..7, word t of the layer's root.
+  uint32_t root_word = 0;
+  if (t < 8) {
+    digest[t] = c->digest[t];
+    root_word = reinterpret_cast<const uint32_t*>(p.tree[p.k0] + (2ull * (1u << (p.L - 1 - p.k0)) - 2) * 32)[t];
+  }
+  // Every CTA has read the state before CTA 0's first channel step overwrites it in device memory, and
+  // every CTA runs before another one writes into its shared memory.
+  cluster.sync();
   bool local = false;  // this layer's values are in vals
   for (uint32_t k = p.k0; k < p.n_inner; ++k) {
     const uint32_t lg = p.L - 1 - k;
