@@ -154,7 +154,7 @@ struct FriChannelDev {
 // mixRoot(root) (src/core/vcs_lifted/blake2_merkle.zig:236-247), then drawSecureFelt
 // (src/core/channel/blake2s.zig:52-112,260-279) into alpha[slot]; the root is kept in roots[slot].
 cudaError_t fri_channel_step(FriChannelDev* c, const uint8_t* root, uint32_t slot, cudaStream_t stream);
-// The inner FRI layers from line layer fri_tail_first(L, n_inner) on (at most 2^13 values each) in one
+// The inner FRI layers from line layer fri_tail_first(L, n_inner) on (at most 2^12 values each) in one
 // cluster: per layer the channel step, the fold and the next layer's commitment, in the order and with
 // the outputs of fri_channel_step + fri_fold_commit. line[k]: line layer k (4 coordinate columns of
 // 2^(L-1-k)); trees[k]: its tree; line[n_inner] receives the last layer.

@@ -252,10 +252,13 @@ __global__ void __launch_bounds__(NODE_THREADS) k_merkle_nodes(uint8_t* layers, 
 // issue one G step each per half round; between the column and the diagonal steps a, c and d move to
 // the neighbour lanes and b, the last word a G step completes, stays, so the shuffles hide behind the
 // steps around them. About 1.0 us a level. It takes 1.4 times
-// the instructions per hash, so levels of more than 128 parents per CTA, which keep a multiprocessor
+// the instructions per hash, so levels of more than 64 parents per CTA, which keep a multiprocessor
 // busy, stay with one lane per hash. (The rounds as a loop, with the offsets in shared memory, took
 // 1.65 us a level: the loads and the loop lengthen the chain.)
-constexpr uint32_t QUAD_THREADS = 512;
+// 256 threads at 80 registers: with 512 at 128 a CTA needs an empty multiprocessor, and a cluster eight of them at
+// once, which other proofs' grinds seldom leave (a batch of 16 proofs with eight in flight then took 53 or 69 ms
+// from one run to the next; single proofs were up to 2% faster).
+constexpr uint32_t QUAD_THREADS = 256;
 constexpr uint32_t QCAP = 512;             // hashes per buffer
 constexpr uint32_t QS = QCAP + 8;          // word stride: word w of hash i at w * QS + i; 8 extra words
                                            // put the four lanes of a hash on different banks
@@ -399,8 +402,8 @@ __device__ __forceinline__ uint32_t quad_fold(QuadBuffers& sm, const QuadLane& L
 // The top of a tree, the layers above 2^child_log children (child_log <= 12), in one launch: one CTA up
 // to 2^9 children, above that a cluster of 2, 4 or 8 CTAs, each folding 512 children to one node;
 // every CTA sends its node to CTA 0's shared memory, which folds the last levels. 2^12 children took
-// 14.2 us in eight CTAs plus 5.5 us and a launch in one with one lane per hash; now 16.7 us.
-__global__ void __launch_bounds__(QUAD_THREADS) k_merkle_top(uint8_t* layers, uint32_t max_log, uint32_t child_log,
+// 14.2 us in eight CTAs plus 5.5 us and a launch in one with one lane per hash; in CTAs of 512 threads 16.7 us.
+__global__ void __launch_bounds__(QUAD_THREADS, 3) k_merkle_top(uint8_t* layers, uint32_t max_log, uint32_t child_log,
                                                              Seeds seeds, uint32_t one) {
   __shared__ __align__(16) QuadBuffers sm;
   __shared__ uint32_t top[8][8];
@@ -562,8 +565,8 @@ __global__ void __launch_bounds__(32) k_fri_channel(FriChannelDev* c, const uint
 // part of the tree to one node; the eight nodes are sent to every CTA, and each folds the last three
 // levels and runs the channel step itself, so a layer needs one cluster barrier. Layers of fewer than
 // 128 folded values run in CTA 0 alone. One CTA of 1024 threads with one lane per hash took
-// 158 us for the layers from 2^12 on, after 27 us and three launches for the 2^13 one; now 127 us for all.
-constexpr uint32_t FRI_TAIL_LOG = 13, FRI_TAIL_CTAS = 8;
+// 158 us for the layers from 2^12 on; with CTAs of 512 threads 99 us, now about as much.
+constexpr uint32_t FRI_TAIL_LOG = 12, FRI_TAIL_CTAS = 8;
 struct FriTailParams {
   uint32_t L, k0, n_inner;
   uint32_t* line[FRI_MAX_LAYERS + 1];
@@ -572,7 +575,7 @@ struct FriTailParams {
   Seeds seeds;
 };
 
-__global__ void __launch_bounds__(QUAD_THREADS) k_fri_tail(FriChannelDev* c, const __grid_constant__ FriTailParams p,
+__global__ void __launch_bounds__(QUAD_THREADS, 3) k_fri_tail(FriChannelDev* c, const __grid_constant__ FriTailParams p,
                                                            uint32_t one) {
   constexpr uint32_t VALS = 1u << (FRI_TAIL_LOG - 1 - 3);  // folded values of one CTA
   static_assert(VALS <= QUAD_THREADS && VALS <= QCAP, "one thread and one leaf per value");

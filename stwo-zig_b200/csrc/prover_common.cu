@@ -38,7 +38,7 @@ int32_t fri_pow_queries(const DeviceTables& T, int sm_count, Channel& ch, const 
     // commits it in the same launch sequence.
     SB_CKE(fri_fold_commit(T, true, L, fb.quot, NL, &fb.chan->alpha[0], fb.line[0], 1ull << (L - 1),
                           n_inner > 0 ? fb.line_tree[0] : nullptr, fs));
-    // Large layers one launch sequence each; the small ones (at most 2^13 values) in one launch.
+    // Large layers one launch sequence each; the small ones (at most 2^12 values) in one launch.
     const uint32_t k_tail = fri_tail_first(L, n_inner);
     for (uint32_t k = 0; k < k_tail; ++k) {
       uint32_t lg = L - 1 - k;
