@@ -402,7 +402,7 @@ __device__ __forceinline__ uint32_t quad_fold(QuadBuffers& sm, const QuadLane& L
 // The top of a tree, the layers above 2^child_log children (child_log <= 12), in one launch: one CTA up
 // to 2^9 children, above that a cluster of 2, 4 or 8 CTAs, each folding 512 children to one node;
 // every CTA sends its node to CTA 0's shared memory, which folds the last levels. 2^12 children took
-// 14.2 us in eight CTAs plus 5.5 us and a launch in one with one lane per hash; in CTAs of 512 threads 16.7 us.
+// 14.2 us in eight CTAs plus 5.5 us and a launch in one with one lane per hash; in CTAs of 512 threads 16.7 us, now 19-26 us.
 __global__ void __launch_bounds__(QUAD_THREADS, 3) k_merkle_top(uint8_t* layers, uint32_t max_log, uint32_t child_log,
                                                              Seeds seeds, uint32_t one) {
   __shared__ __align__(16) QuadBuffers sm;
@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(32) k_fri_channel(FriChannelDev* c, const uint
 // part of the tree to one node; the eight nodes are sent to every CTA, and each folds the last three
 // levels and runs the channel step itself, so a layer needs one cluster barrier. Layers of fewer than
 // 128 folded values run in CTA 0 alone. One CTA of 1024 threads with one lane per hash took
-// 158 us for the layers from 2^12 on; with CTAs of 512 threads 99 us, now about as much.
+// 158 us for the layers from 2^12 on; with CTAs of 512 threads 99 us, now 121 us.
 constexpr uint32_t FRI_TAIL_LOG = 12, FRI_TAIL_CTAS = 8;
 struct FriTailParams {
   uint32_t L, k0, n_inner;
