@@ -974,9 +974,17 @@ cudaError_t interpolate_extend(const DeviceTables& t, uint32_t log_size, uint32_
     p.do_inverse = 1; p.itv = t.view(log_size, true); p.scale = inv_pow2(log_size); p.coef = coeffs; p.cs = co_stride;
     p.do_forward = 1; p.ftv = t.view(out_log, false); p.copies = 1u << log_blowup; p.out = lde; p.os = lde_stride;
     const uint64_t n = 1ull << log_size, m = 1ull << out_log;
-    return launch_small(log_size, p, n_cols,
-                        overlap(evals, ev_stride, n, coeffs, co_stride, n, n_cols) ||
-                            overlap(evals, ev_stride, n, lde, lde_stride, m, n_cols), stream);
+    const bool on_lde = overlap(evals, ev_stride, n, lde, lde_stride, m, n_cols);
+    // One launch orders a column's reads before its own writes only. Evaluations in the lde buffer other than
+    // column on column (packed at its front, say) would be overwritten by the CTAs of other columns, and
+    // coefficients stored there belong under the evaluations: then all coefficients first.
+    if ((on_lde && (evals != lde || ev_stride != lde_stride)) || overlap(coeffs, co_stride, n, lde, lde_stride, m, n_cols)) {
+      p.do_forward = 0;
+      const cudaError_t e = launch_small(log_size, p, n_cols, true, stream);
+      if (e != cudaSuccess) return e;
+      return extend(t, log_size, log_blowup, n_cols, coeffs, co_stride, lde, lde_stride, stream);
+    }
+    return launch_small(log_size, p, n_cols, on_lde || overlap(evals, ev_stride, n, coeffs, co_stride, n, n_cols), stream);
   }
   if (use16(log_size, out_log, evals, ev_stride, lde, lde_stride) && aligned16(coeffs, co_stride)) {
     // Variant 0: the fused high pass (blow-up 2, 2^17 .. 2^22); variant 1: the generic one.

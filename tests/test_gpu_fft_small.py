@@ -55,3 +55,32 @@ def test_in_place(ctx, log, pad, offset):
     ctx.evaluate(t, log, 3, stride)
     got = _get(t, 3, stride)
     assert np.array_equal(got[:, : 1 << log], cols) and (got[:, 1 << log :] == 0x5A5A5A5A).all()
+
+
+@pytest.mark.parametrize("log,blowup", [(8, 1), (9, 1), (10, 2), (11, 1), (12, 2), (13, 1), (14, 1), (14, 2), (15, 1)])
+@pytest.mark.parametrize("place", ["front", "middle", "back"])
+def test_evaluations_in_the_lde_buffer(ctx, log, blowup, place):
+    """Evaluations packed anywhere in the buffer that receives their extension, more columns than CTAs run at once."""
+    import torch
+    n, size, words = 700, 1 << log, 700 << (log + blowup)
+    cols = torch.from_numpy(np.random.default_rng(log).integers(0, P, size=(n, size), dtype=np.uint32).view(np.int32)).cuda()
+    co, ref = torch.empty_like(cols), torch.empty(words, dtype=torch.int32, device="cuda")
+    ctx.interpolate_and_extend(cols, co, ref, log, blowup, n)
+    lde, co2 = torch.empty_like(ref), torch.empty_like(co)
+    at = {"front": 0, "middle": (words - cols.numel()) // 2 + 4, "back": words - cols.numel()}[place]
+    evals = lde[at : at + cols.numel()]
+    evals.copy_(cols.view(-1))
+    ctx.interpolate_and_extend(evals, co2, lde, log, blowup, n)
+    assert torch.equal(co, co2) and torch.equal(ref, lde)
+
+
+@pytest.mark.parametrize("log", [11, 12, 13, 14])
+def test_coefficients_in_the_lde_buffer(ctx, log):
+    """One column whose coefficients go where its second blown-up block comes: the extension stands at the end."""
+    import torch
+    ev = _buf(np.random.default_rng(log).integers(0, P, size=(1, 1 << log), dtype=np.uint32), 1 << log)
+    co, ref = torch.empty_like(ev), torch.empty(2 << log, dtype=torch.int32, device="cuda")
+    ctx.interpolate_and_extend(ev, co, ref, log, 1, 1)
+    lde = torch.empty_like(ref)
+    ctx.interpolate_and_extend(ev, lde[1 << log :], lde, log, 1, 1)
+    assert torch.equal(ref, lde)
