@@ -242,7 +242,9 @@ int32_t stwo_b200_evaluate_columns(stwo_b200_context* ctx, uint32_t log_size, ui
                                    uint64_t stride, void* stream);
 /* Evaluations on CanonicCoset(log_size) -> coefficients and evaluations on
  * CanonicCoset(log_size + log_blowup), fused. Replaces interpolateAndEvaluateCircleBuffers
- * (src/backends/cpu_scalar/mod.zig:185-266, src/prover/pcs/columns/preparation.zig:212-352). */
+ * (src/backends/cpu_scalar/mod.zig:185-266, src/prover/pcs/columns/preparation.zig:212-352).
+ * coeffs may be evals (the same stride), and evals may lie anywhere in the lde buffer: every evaluation has
+ * been read before an extension is written over it. */
 int32_t stwo_b200_interpolate_and_extend(stwo_b200_context* ctx, uint32_t log_size, uint32_t log_blowup,
                                          uint32_t n_cols, const uint32_t* evals, uint64_t evals_stride,
                                          uint32_t* coeffs, uint64_t coeffs_stride, uint32_t* lde,

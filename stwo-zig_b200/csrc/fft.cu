@@ -1003,8 +1003,10 @@ cudaError_t interpolate_extend(const DeviceTables& t, uint32_t log_size, uint32_
       return launch_low12(t, false, out_log, n_cols, lde, lde_stride, lde, lde_stride, 0, stream);
     };
     const bool fusable = log_blowup == 1 && log_size - B12 >= 5;
-    // The chain reads evals only, so it can run again for timing unless evals is also an output.
-    const bool rerunnable = evals != coeffs && evals != lde;
+    // The chain reads evals only, so it can run again for timing unless an output overlaps them.
+    const uint64_t n = 1ull << log_size;
+    const bool rerunnable = !overlap(evals, ev_stride, n, coeffs, co_stride, n, n_cols) &&
+                            !overlap(evals, ev_stride, n, lde, lde_stride, 1ull << out_log, n_cols);
     return tuned_run(TUNE_LDE1, log_size, n_cols, fusable ? 2 : 1, rerunnable, stream, chain);
   }
   const uint32_t b = std::min(log_size, LOW_BITS);

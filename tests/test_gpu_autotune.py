@@ -81,3 +81,19 @@ def test_tuning_records_each_variant_and_keeps_the_fastest(ctx, forced):
     e = entries[0]
     assert e["ms"][0] > 0 and e["ms"][1] > 0
     assert e["ms"][e["variant"]] == min(e["ms"][:2])
+
+
+@pytest.mark.parametrize("log,n,place", [(17, 7, "front"), (17, 6, "back"), (18, 5, "middle")])
+def test_first_call_with_evaluations_in_the_lde_buffer(ctx, log, n, place):
+    """A key's first call runs several variants only where a run leaves the evaluations as they were."""
+    import torch
+    cols = np.random.default_rng(log + n).integers(0, P, size=(n, 1 << log), dtype=np.uint32)
+    lde, coeffs = torch.empty(n << (log + 1), dtype=torch.int32, device="cuda"), torch.empty(n << log, dtype=torch.int32, device="cuda")
+    at = {"front": 0, "middle": n << (log - 1), "back": n << log}[place]
+    evals = lde[at : at + (n << log)]
+    evals.copy_(_dev(cols).view(-1))
+    ctx.interpolate_and_extend(evals, coeffs, lde, log, 1, n)
+    co, le = _host(coeffs).reshape(n, -1), _host(lde).reshape(n, -1)
+    for c in (0, n - 1):
+        ref = oracle.interpolate(cols[c])
+        assert np.array_equal(co[c], ref) and np.array_equal(le[c], oracle.extend(ref, 1)), c
