@@ -1101,9 +1101,10 @@ cudaError_t accumulate_quotients(const DeviceTables& t, uint32_t log_size, uint3
     return cudaGetLastError();
   }
   // The bulk-staged kernel takes whole 512-row tiles of 16-byte aligned columns (the caller vouches
-  // for the pointers by passing `status`). It runs when a caller forces the last variant.
+  // for the pointers by passing `status`) and stores two words at a time. It runs when a caller forces the
+  // last variant.
   const bool bulk = status != nullptr && log_size >= 16 && n_batches <= QB_MAX_BATCHES &&
-                    n_entries <= QUOT_MAX_ENTRIES;
+                    n_entries <= QUOT_MAX_ENTRIES && (reinterpret_cast<uintptr_t>(out) & 7) == 0 && out_stride % 2 == 0;
   auto run = [&](int variant) -> cudaError_t {
     const PointTable pts{t.points};
     if (variant == 3 && bulk) {

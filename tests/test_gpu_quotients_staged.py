@@ -95,6 +95,22 @@ def test_quotient_op_variants_equal_the_register_kernel(ctx, n_cols):
     del cols
 
 
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_forced_staged_kernel_with_an_unaligned_output(ctx, staged, offset):
+    """The staged kernel stores two words at a time: it leaves an output off its 8-byte alignment to the other one."""
+    import stwo_b200 as sb
+    import torch
+    log, n_cols = 16, 9
+    cols, ptrs, coeffs, (px, py, sa, sbb) = _quotient_case(n_cols, log)
+    out = torch.full(((4 << log) + offset,), -1, dtype=torch.int32, device="cuda")
+    ctx.accumulate_quotients(log, ptrs, coeffs, px, py, sa, sbb, out[offset:], n_cols)
+    sb.autotune_mode(-1)
+    ref = torch.empty(4 << log, dtype=torch.int32, device="cuda")
+    ctx.accumulate_quotients(log, ptrs, coeffs, px, py, sa, sbb, ref, n_cols)
+    assert torch.equal(out[offset:], ref) and (out[:offset] == -1).all()
+    del cols
+
+
 def test_staged_wait_that_runs_out_fails_the_proof_and_the_context_stays_usable(ctx, staged):
     import stwo_b200 as sb
     o, g = _cfg("functional")
