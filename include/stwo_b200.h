@@ -485,6 +485,11 @@ int32_t stwo_b200_arm_allocation_failure_for_testing(uint32_t nth);
  * faults and no wait is unbounded; the context stays usable. */
 int32_t stwo_b200_arm_quotient_stage_timeout_for_testing(void);
 
+/* Runs the shared-memory set-up that stwo_b200_context_create does on its device (one attribute per kernel
+ * that takes more than 48 KB) against a counter in place of the device: the kernels set, the largest size,
+ * and, with fail_at > 0, the error of the fail_at-th one. Needs no GPU. */
+int32_t stwo_b200_count_smem_limits_for_testing(uint32_t fail_at, uint32_t* n_kernels, uint32_t* largest);
+
 #ifdef __cplusplus
 }
 #endif

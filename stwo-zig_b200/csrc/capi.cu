@@ -683,6 +683,15 @@ int32_t stwo_b200_arm_allocation_failure_for_testing(uint32_t nth) {
   return STWO_B200_OK;
 }
 
+int32_t stwo_b200_count_smem_limits_for_testing(uint32_t fail_at, uint32_t* n_kernels, uint32_t* largest) {
+  if (!n_kernels || !largest) return set_error(STWO_B200_E_INVALID, "null count");
+  *n_kernels = *largest = 0;
+  return cuda_status(sb::kernel_smem_limits([&](const void* kernel, int bytes) {
+                       *largest = std::max(*largest, (uint32_t)bytes);
+                       return kernel && ++*n_kernels != fail_at ? cudaSuccess : cudaErrorInvalidValue;
+                     }), "shared memory limit");
+}
+
 int32_t stwo_b200_server_snapshot_get(stwo_b200_server* server, stwo_b200_server_snapshot* out) {
   if (!server || !out) return set_error(STWO_B200_E_INVALID, "null server argument");
   sb::ServerSnapshot s = server->server->snapshot();

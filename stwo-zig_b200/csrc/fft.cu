@@ -682,6 +682,20 @@ inline uint32_t inv_pow2(uint32_t log) { return minv(1u << log); }
 
 }  // namespace
 
+cudaError_t fft_smem_limits(const SetSmemLimit& set) {
+  struct { const void* kernel; size_t bytes; } const limits[] = {
+      {(const void*)k_fft_high, 200 * 1024},
+      {(const void*)k_fft_high16<1024, 1>, 64 * 1024},
+      {(const void*)k_fft_high16_lde1<9>, (size_t)64 << 10},
+      {(const void*)k_fft_high16_lde1<10>, (size_t)64 << 11},
+      {(const void*)k_fft_small<14>, (size_t)4 << 14}};
+  for (const auto& l : limits) {
+    const cudaError_t e = set(l.kernel, (int)l.bytes);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 TwiddleView DeviceTables::view(uint32_t domain_log, bool inverse) const {
   TwiddleView v;
   v.tower = inverse ? itw : tw;
@@ -724,11 +738,6 @@ static cudaError_t launch_low(const DeviceTables& t, bool inverse, uint32_t doma
 static cudaError_t launch_high(const HighParams& p, uint32_t n_cols, cudaStream_t stream) {
   uint32_t rows_log = std::max(p.src_log, p.do_forward ? p.out_log : p.src_log) - p.b;
   size_t smem = ((size_t)HIGH_T * 4) << rows_log;
-  static const bool attr_set = [] {  // once per process (thread-safe static initialisation)
-    cudaFuncSetAttribute(k_fft_high, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    return true;
-  }();
-  (void)attr_set;
   dim3 grid((1u << p.b) / HIGH_T, n_cols);
   k_fft_high<<<grid, HIGH_THREADS, smem, stream>>>(p); note_launch();
   return cudaGetLastError();
@@ -793,12 +802,6 @@ static cudaError_t launch_low12(const DeviceTables& t, bool inverse, uint32_t do
 static cudaError_t launch_high16(const High16Params& p, uint32_t n_cols, cudaStream_t stream) {
   uint32_t rows = p.do_forward ? std::max(p.rows_in, p.rows_out) : p.rows_in;
   size_t smem = (size_t)64 << rows;
-  static const bool attr_set = [] {  // once per process (thread-safe static initialisation)
-    cudaFuncSetAttribute(k_fft_high16<512, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * 1024);
-    cudaFuncSetAttribute(k_fft_high16<1024, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-    return true;
-  }();
-  (void)attr_set;
   dim3 grid(1u << (B12 - 4), n_cols);
   if (rows <= 9) k_fft_high16<512, 3><<<grid, 1u << rows, smem, stream>>>(p);
   else k_fft_high16<1024, 1><<<grid, 1u << rows, smem, stream>>>(p);
@@ -809,11 +812,6 @@ static cudaError_t launch_high16(const High16Params& p, uint32_t n_cols, cudaStr
 template <int R>
 static cudaError_t launch_lde1_rows(const High16Params& p, uint32_t n_cols, cudaStream_t stream) {
   const size_t smem = (size_t)64 << (R + 1);
-  static const bool attr_set = [] {  // once per process (thread-safe static initialisation)
-    cudaFuncSetAttribute(k_fft_high16_lde1<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((size_t)64 << (R + 1)));
-    return true;
-  }();
-  (void)attr_set;
   k_fft_high16_lde1<R><<<dim3(1u << (B12 - 4), n_cols), 1u << R, smem, stream>>>(p);
   note_launch();
   return cudaGetLastError();
@@ -833,11 +831,6 @@ static cudaError_t launch_high16_lde1(const High16Params& p, uint32_t n_cols, cu
 
 template <int N>
 static cudaError_t launch_small_n(const SmallParams& p, dim3 grid, cudaStream_t stream) {
-  static const bool attr_set = [] {  // once per process (thread-safe static initialisation)
-    cudaFuncSetAttribute(k_fft_small<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 << N);
-    return true;
-  }();
-  (void)attr_set;
   k_fft_small<N><<<grid, 1u << (N - 4), 4u << N, stream>>>(p);
   note_launch();
   return cudaGetLastError();

@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <functional>
 
 #include "circle.cuh"
 #include "field.cuh"
@@ -35,6 +36,16 @@ struct DeviceTables {
 
 // Builds the twiddle towers for root log R on the device (one-time).
 cudaError_t build_twiddle_tower(DeviceTables& t, uint32_t root_log, cudaStream_t stream);
+
+// Calls `set` for every kernel that takes more than 48 KB of dynamic shared memory, with its largest size, and
+// returns the first error. The limit belongs to the device, so a context sets them all when it is made.
+using SetSmemLimit = std::function<cudaError_t(const void* kernel, int bytes)>;
+cudaError_t fft_smem_limits(const SetSmemLimit& set);
+cudaError_t prover_smem_limits(const SetSmemLimit& set);
+inline cudaError_t kernel_smem_limits(const SetSmemLimit& set) {
+  const cudaError_t e = fft_smem_limits(set);
+  return e != cudaSuccess ? e : prover_smem_limits(set);
+}
 
 // ---- Circle FFT (src/prover/poly/circle/transforms.zig) -------------------
 // In-place forward (evaluate) or inverse (interpolate, scaled by 1/n) transform

@@ -142,6 +142,10 @@ int32_t Context::init(int dev, uint32_t tower_log) {
   if (cudaSetDevice(dev) != cudaSuccess) return E_CUDA;
   cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
   tables.sm_count = (uint32_t)std::max(sm_count, 1);
+  if (kernel_smem_limits([](const void* kernel, int bytes) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+      }) != cudaSuccess)
+    return E_CUDA;
   if (cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) != cudaSuccess) return E_CUDA;
   // Keep freed stream-ordered allocations cached in this process's default pool
   // instead of returning them to the driver at every synchronization.

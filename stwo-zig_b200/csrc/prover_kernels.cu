@@ -958,7 +958,26 @@ inline uint32_t grid_for(uint64_t n, uint32_t threads, uint32_t cap = 148 * 32) 
   return g == 0 ? 1 : (uint32_t)g;
 }
 
+// Largest dynamic shared memory of the kernels that take more than the 48 KB a launch has without asking.
+constexpr size_t COMP_SMEM_MAX = mma_ring_bytes(COMP_STAGES) + 3008 * 32;  // W <= 3000
+constexpr size_t QUOT_SMEM_MAX = 200 * 1024;
+constexpr size_t QB_SMEM_MAX = (size_t)QB_STAGES * QB_GROUP * QB_ROWS * 4 +
+                               (size_t)QUOT_MAX_ENTRIES * (16 + sizeof(void*)) +
+                               (size_t)(QUOT_MAX_ENTRIES / QB_GROUP + QB_MAX_BATCHES) * sizeof(QbItem);
+
 }  // namespace
+
+cudaError_t prover_smem_limits(const SetSmemLimit& set) {
+  struct { const void* kernel; size_t bytes; } const limits[] = {
+      {(const void*)k_composition_mma<true>, COMP_SMEM_MAX},  {(const void*)k_composition_mma<false>, COMP_SMEM_MAX},
+      {(const void*)k_quotients_mma<true>, QUOT_SMEM_MAX},    {(const void*)k_quotients_mma<false>, QUOT_SMEM_MAX},
+      {(const void*)k_quotients_bulk<2>, QB_SMEM_MAX},        {(const void*)k_quotients_bulk<3>, QB_SMEM_MAX}};
+  for (const auto& l : limits) {
+    const cudaError_t e = set(l.kernel, (int)l.bytes);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
 
 cudaError_t quadratic_trace(uint32_t log_n, uint32_t W, const uint32_t recipe[7], uint32_t* out, uint64_t stride,
                             cudaStream_t stream) {
@@ -991,13 +1010,6 @@ cudaError_t wide_fib_composition(uint32_t log_n, uint32_t W, const uint32_t* eva
   const uint32_t grid = std::min<uint32_t>((blocks + per_cta - 1) / per_cta, 148 * 4);
   const size_t smem_m = (size_t)mma_ring_bytes(COMP_STAGES) + (size_t)((W + 7) / 8) * 8 * 32;
   auto kernel = aligned ? k_composition_mma<true> : k_composition_mma<false>;
-  static const bool attr = [] {  // once per process (thread-safe static initialisation); W <= 3000
-    constexpr int kMax = (int)mma_ring_bytes(COMP_STAGES) + 3008 * 32;
-    cudaFuncSetAttribute(k_composition_mma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax);
-    cudaFuncSetAttribute(k_composition_mma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax);
-    return true;
-  }();
-  (void)attr;
   kernel<<<grid, MMA_THREADS, smem_m, stream>>>(log_n, W, eval, stride, coeffs_dev, den_inv0, den_inv1, out, out_stride);
   note_launch();
   return cudaGetLastError();
@@ -1074,26 +1086,13 @@ cudaError_t accumulate_quotients(const DeviceTables& t, uint32_t log_size, uint3
   // Tensor-core kernel: every batch padded to a multiple of eight entries.
   const uint32_t padded = n_entries + 7 * n_batches;
   const size_t smem_m = (size_t)mma_ring_bytes(QUOT_STAGES) + (size_t)padded * (16 + sizeof(void*));
-  constexpr size_t SMEM_M_MAX = 200 * 1024;
   // Bulk-staged kernel: the ring, the coefficients and pointers, and the item table (every batch
   // adds at most one partial group).
   const uint32_t item_cap = (n_entries + QB_GROUP - 1) / QB_GROUP + n_batches;
   const size_t smem_b = (size_t)QB_STAGES * QB_GROUP * QB_ROWS * 4 + (size_t)n_entries * (16 + sizeof(void*)) +
                         (size_t)item_cap * sizeof(QbItem);
-  constexpr size_t SMEM_B_MAX = (size_t)QB_STAGES * QB_GROUP * QB_ROWS * 4 +
-                                (size_t)QUOT_MAX_ENTRIES * (16 + sizeof(void*)) +
-                                (size_t)(QUOT_MAX_ENTRIES / QB_GROUP + QB_MAX_BATCHES) * sizeof(QbItem);
-  static const bool attr = [&] {  // once per process (thread-safe static initialisation)
-    cudaFuncSetAttribute(k_quotients, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_quotients_mma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_M_MAX);
-    cudaFuncSetAttribute(k_quotients_mma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_M_MAX);
-    cudaFuncSetAttribute(k_quotients_bulk<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_B_MAX);
-    cudaFuncSetAttribute(k_quotients_bulk<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_B_MAX);
-    return true;
-  }();
-  (void)attr;
   // The tensor-core kernel takes whole blocks of 64 rows.
-  if ((1ull << log_size) < MMA_ROWS || smem_m > SMEM_M_MAX) {
+  if ((1ull << log_size) < MMA_ROWS || smem_m > QUOT_SMEM_MAX) {
     k_quotients<<<grid_for(1ull << log_size, 256), 256, smem, stream>>>(PointTable{t.points}, log_size, n_batches, batches,
                                                                         one ? *one : QuotientBatchDev{}, col_ptrs,
                                                                         coeff_c, out, out_stride);

@@ -135,6 +135,7 @@ _SIGS = {
     "stwo_b200_server_set_request_timeout": [_vp, _u32],
     "stwo_b200_arm_allocation_failure_for_testing": [_u32],
     "stwo_b200_arm_quotient_stage_timeout_for_testing": [],
+    "stwo_b200_count_smem_limits_for_testing": [_u32, ctypes.POINTER(_u32), ctypes.POINTER(_u32)],
     "stwo_b200_autotune_mode": [_i32],
     "stwo_b200_autotune_wide_fibonacci": [_vp, _u32, _u32, _u32],
     "stwo_b200_autotune_table": [_vp, ctypes.c_size_t, ctypes.POINTER(ctypes.c_size_t)],
@@ -614,6 +615,14 @@ def arm_quotient_stage_timeout_for_testing() -> None:
     """Makes the next bulk-staged quotient launch leave its first stage empty: its bounded waits run
     out (about a second), and the proof or op fails with E_CUDA; no GPU fault is involved."""
     _check(_lib.stwo_b200_arm_quotient_stage_timeout_for_testing())
+
+
+def count_smem_limits_for_testing(fail_at: int = 0) -> tuple[int, int]:
+    """The kernels whose shared memory limit a new context raises on its device, and the largest one, against a
+    counter in place of the device (no GPU needed); the fail_at-th one fails."""
+    n, largest = _u32(0), _u32(0)
+    _check(_lib.stwo_b200_count_smem_limits_for_testing(fail_at, ctypes.byref(n), ctypes.byref(largest)))
+    return n.value, largest.value
 
 
 AUTOTUNE_OPS = {0: "interpolate+extend high pass (fused, generic)", 1: "Merkle leaves (5, 6, 4 CTAs/SM)",

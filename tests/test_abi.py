@@ -40,3 +40,16 @@ def test_status_strings_and_telemetry_without_device():
     assert stwo_b200.lib().stwo_b200_status_string(stwo_b200.E_CONSTRAINTS) == b"constraints not satisfied"
     assert stwo_b200.lib().stwo_b200_version().startswith(b"stwo_b200")
     assert stwo_b200.kernel_launches() >= 0
+
+
+def test_every_context_raises_the_shared_memory_limits():
+    """The limits belong to a device: the second context's set-up does what the first one's did, and a limit that
+    cannot be set is an error."""
+    import pytest
+    import stwo_b200
+    first = stwo_b200.count_smem_limits_for_testing()
+    assert first[0] >= 11 and first[1] > 48 * 1024 and stwo_b200.count_smem_limits_for_testing() == first
+    for k in (1, first[0]):
+        with pytest.raises(stwo_b200.StwoError):
+            stwo_b200.count_smem_limits_for_testing(k)
+    assert stwo_b200.count_smem_limits_for_testing() == first

@@ -324,3 +324,4 @@ pub extern fn stwo_b200_autotune_table(out: ?[*]TuneEntry, cap: usize, n: *usize
 
 pub extern fn stwo_b200_arm_allocation_failure_for_testing(nth: u32) i32;
 pub extern fn stwo_b200_arm_quotient_stage_timeout_for_testing() i32;
+pub extern fn stwo_b200_count_smem_limits_for_testing(fail_at: u32, n_kernels: *u32, largest: *u32) i32;
