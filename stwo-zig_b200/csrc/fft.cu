@@ -650,14 +650,19 @@ __global__ void __launch_bounds__(1 << (N - 4), N == 14 ? 1 : 512 >> (N - 4)) k_
   if (!p.do_forward) return;
   for (uint32_t copy = blockIdx.z; copy < p.copies; copy += gridDim.z) {
     const uint32_t block = copy << N;
+    // 1024 threads have 64 registers each: the windows' addresses are formed again for every copy (kept across
+    // the copies they spilled 352 bytes; one column of 2^14 took 17.1 us, now 11.0, and 4000 take 246 instead of
+    // 418 us). Smaller columns keep them (128 registers; formed again they take up to 7% longer).
+    uint32_t tc = th;
+    if (N == 14) asm volatile("" : "+r"(tc));
     uint32_t y[16];
 #pragma unroll
     for (int k = 0; k < 16; ++k) y[k] = x[k];
-    radix16<false, 0, 4, fft16::RANGE_CANON>(y, p.ftv, 0, TOP, block | th);
+    radix16<false, 0, 4, fft16::RANGE_CANON>(y, p.ftv, 0, TOP, block | tc);
 #pragma unroll
     for (int i = NW - 2; i >= 0; --i) {
-      const uint32_t v0 = win_w0<N>(i + 1), from = swz(spread(th, v0));
-      const uint32_t w0 = win_w0<N>(i), base = spread(th, w0), to = swz(base);
+      const uint32_t v0 = win_w0<N>(i + 1), from = swz(spread(tc, v0));
+      const uint32_t w0 = win_w0<N>(i), base = spread(tc, w0), to = swz(base);
       __syncthreads();  // the words exchanged before have been read
 #pragma unroll
       for (int k = 0; k < 16; ++k) sm[from ^ swz((uint32_t)k << v0)] = y[k];
@@ -667,12 +672,12 @@ __global__ void __launch_bounds__(1 << (N - 4), N == 14 ? 1 : 512 >> (N - 4)) k_
       radix16_dyn<false>(y, p.ftv, 0, w0, block | base, win_nl<N>(i));
     }
     // The thread's 16 consecutive words leave through shared memory, so that the stores are contiguous.
-    const uint32_t a = swz(th << 4), c = swz(th);
+    const uint32_t a = swz(tc << 4), c = swz(tc);
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 16; ++k) sm[a ^ swz((uint32_t)k)] = fft16::canon_s(y[k]);
     __syncthreads();
-    uint32_t* out = p.out + col * p.os + block + th;
+    uint32_t* out = p.out + col * p.os + block + tc;
 #pragma unroll
     for (int k = 0; k < 16; ++k) out[k * T] = sm[c ^ swz((uint32_t)k << TOP)];
   }
