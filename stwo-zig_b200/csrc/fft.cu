@@ -848,11 +848,18 @@ static bool overlap(const uint32_t* a, uint64_t sa, uint64_t wa, const uint32_t*
   return a < eb && b < ea;
 }
 // `shared`: an output overlaps the source, so one CTA reads a column before it writes anything.
-static cudaError_t launch_small(uint32_t log, SmallParams p, uint32_t n_cols, bool shared, cudaStream_t stream) {
+static cudaError_t launch_small(const DeviceTables& t, uint32_t log, SmallParams p, uint32_t n_cols, bool shared,
+                                cudaStream_t stream) {
   // A CTA per blown-up copy while that keeps to about two CTAs per multiprocessor: beyond, interpolating
-  // once per column is less work.
-  const bool split = p.do_forward && p.copies > 1 && !shared && (uint64_t)n_cols * p.copies <= 296;
-  const dim3 grid(1, n_cols, split ? p.copies : 1);
+  // once per column is less work. Copies too many for that are shared out over CTAs as far as columns leave
+  // multiprocessors without one (37 columns of 2^14 extended by 16: 126 us with a CTA per column, 36 with four).
+  uint32_t z = 1;
+  if (p.do_forward && !shared) {
+    if ((uint64_t)n_cols * p.copies <= 2 * t.sm_count) z = p.copies;
+    else
+      while (2 * z <= p.copies && 2ull * z * n_cols <= t.sm_count) z *= 2;
+  }
+  const dim3 grid(1, n_cols, z);
   switch (log) {
     case 9: return launch_small_n<9>(p, grid, stream);
     case 10: return launch_small_n<10>(p, grid, stream);
@@ -874,7 +881,7 @@ cudaError_t fft_columns(const DeviceTables& t, bool inverse, uint32_t log_size, 
     } else {
       p.do_forward = 1; p.ftv = t.view(log_size, false); p.copies = 1; p.out = cols; p.os = stride;
     }
-    return launch_small(log_size, p, n_cols, true, stream);
+    return launch_small(t, log_size, p, n_cols, true, stream);
   }
   if (use16(log_size, log_size, cols, stride, cols, stride)) {
     High16Params p{};
@@ -920,7 +927,7 @@ cudaError_t extend(const DeviceTables& t, uint32_t log_size, uint32_t log_blowup
     SmallParams p{};
     p.src = coeffs; p.ss = co_stride;
     p.do_forward = 1; p.ftv = t.view(out_log, false); p.copies = 1u << log_blowup; p.out = lde; p.os = lde_stride;
-    return launch_small(log_size, p, n_cols,
+    return launch_small(t, log_size, p, n_cols,
                         overlap(coeffs, co_stride, 1ull << log_size, lde, lde_stride, 1ull << out_log, n_cols), stream);
   }
   if (use16(log_size, out_log, coeffs, co_stride, lde, lde_stride)) {
@@ -978,11 +985,11 @@ cudaError_t interpolate_extend(const DeviceTables& t, uint32_t log_size, uint32_
     // coefficients stored there belong under the evaluations: then all coefficients first.
     if ((on_lde && (evals != lde || ev_stride != lde_stride)) || overlap(coeffs, co_stride, n, lde, lde_stride, m, n_cols)) {
       p.do_forward = 0;
-      const cudaError_t e = launch_small(log_size, p, n_cols, true, stream);
+      const cudaError_t e = launch_small(t, log_size, p, n_cols, true, stream);
       if (e != cudaSuccess) return e;
       return extend(t, log_size, log_blowup, n_cols, coeffs, co_stride, lde, lde_stride, stream);
     }
-    return launch_small(log_size, p, n_cols, on_lde || overlap(evals, ev_stride, n, coeffs, co_stride, n, n_cols), stream);
+    return launch_small(t, log_size, p, n_cols, on_lde || overlap(evals, ev_stride, n, coeffs, co_stride, n, n_cols), stream);
   }
   if (use16(log_size, out_log, evals, ev_stride, lde, lde_stride) && aligned16(coeffs, co_stride)) {
     // Variant 0: the fused high pass (blow-up 2, 2^17 .. 2^22); variant 1: the generic one.

@@ -21,7 +21,7 @@ def _get(t, n, stride):
 
 
 @pytest.mark.parametrize("log", [8, 9, 10, 11, 12, 13, 14, 15])
-@pytest.mark.parametrize("n,blowup", [(1, 1), (3, 2), (149, 1), (80, 2)])
+@pytest.mark.parametrize("n,blowup", [(1, 1), (3, 2), (149, 1), (80, 2), (37, 4)])
 def test_interpolate_and_extend(ctx, log, n, blowup):
     import torch
     cols = np.random.default_rng(log + n).integers(0, P, size=(n, 1 << log), dtype=np.uint32)
