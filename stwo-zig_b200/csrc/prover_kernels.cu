@@ -90,31 +90,83 @@ __global__ void k_quadratic_trace(uint32_t log_n, uint32_t W, QuadRecipe q, uint
 // CanonicCoset(n+1), sum_k coeff_k * (c_k - a_k^2 - b_k^2), times the inverse
 // coset vanishing value den_inv[row >> n]. coeff_k = random_coeff^(W-3-k).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_composition(uint32_t log_n, uint32_t W, const uint32_t* __restrict__ eval,
-                                                     uint64_t stride, const QM31* __restrict__ coeffs,
-                                                     uint32_t den0, uint32_t den1, uint32_t* out, uint64_t out_stride) {
-  extern __shared__ uint32_t sco[];  // (W-2) * 4 words
+// R consecutive rows per thread, U columns loaded before they are used (a multiple of three: the sums are folded
+// after every third product), each column squared once (its square is b^2 of one constraint and a^2 of the next).
+// R = 2 needs columns and output aligned to two words (eval, stride, out, out_stride).
+// Bound by the field products where rows are many, by the latency of the loads where they are few: 1000 columns on
+// 16 rows took 116 us a column at a time and 75 us six at a time, 39 us with 24 columns in flight.
+
+template <int R>
+__device__ __forceinline__ void load_rows(const uint32_t* p, uint32_t (&v)[R]) {
+  if (R == 2) {
+    const uint2 x = __ldg(reinterpret_cast<const uint2*>(p));
+    v[0] = x.x; v[R - 1] = x.y;
+  } else {
+    v[0] = __ldg(p);
+  }
+}
+
+template <int R, uint32_t U>
+__global__ void __launch_bounds__(256, U > 6 ? 2 : 4) k_composition(uint32_t log_n, uint32_t W, const uint32_t* __restrict__ eval,
+                                                        uint64_t stride, const QM31* __restrict__ coeffs,
+                                                        uint32_t den0, uint32_t den1, uint32_t* out, uint64_t out_stride) {
+  extern __shared__ uint4 sco[];  // W - 2 coefficients
   const uint32_t n_cons = W - 2;
-  for (uint32_t i = threadIdx.x; i < n_cons; i += blockDim.x) qstore4(coeffs[i], sco + 4 * i);
+  for (uint32_t i = threadIdx.x; i < n_cons; i += blockDim.x) {
+    const QM31 c = coeffs[i];
+    sco[i] = make_uint4(c.c0.a, c.c0.b, c.c1.a, c.c1.b);
+  }
   __syncthreads();
-  const uint32_t rows = 2u << log_n;
-  for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < rows; row += gridDim.x * blockDim.x) {
-    uint32_t a = __ldg(eval + row), b = __ldg(eval + stride + row);
-    uint64_t acc0 = 0, acc1 = 0, acc2 = 0, acc3 = 0;
-    for (uint32_t k = 0; k < n_cons; ++k) {
-      uint32_t c = __ldg(eval + (uint64_t)(k + 2) * stride + row);
-      uint32_t cons = msub(c, madd(mmul(a, a), mmul(b, b)));
-      const uint32_t* q = sco + 4 * k;
-      acc0 += (uint64_t)q[0] * cons; acc1 += (uint64_t)q[1] * cons;
-      acc2 += (uint64_t)q[2] * cons; acc3 += (uint64_t)q[3] * cons;
-      if (k % 3 == 2) { acc0 = mfold64(acc0); acc1 = mfold64(acc1); acc2 = mfold64(acc2); acc3 = mfold64(acc3); }
-      a = b; b = c;
+  const uint32_t groups = (2u << log_n) / R;
+  for (uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x; gi < groups; gi += gridDim.x * blockDim.x) {
+    const uint32_t row0 = gi * R;
+    const uint32_t* p = eval + row0;
+    uint32_t a[R], b[R];  // squares of the two columns before
+    load_rows<R>(p, a);
+    load_rows<R>(p + stride, b);
+    p += 2 * stride;
+    uint64_t acc[R][4];
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      a[j] = mmul(a[j], a[j]);
+      b[j] = mmul(b[j], b[j]);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[j][c] = 0;
     }
-    uint32_t d = (row >> log_n) ? den1 : den0;
-    out[row] = mmul(mreduce64(acc0), d);
-    out[out_stride + row] = mmul(mreduce64(acc1), d);
-    out[2 * out_stride + row] = mmul(mreduce64(acc2), d);
-    out[3 * out_stride + row] = mmul(mreduce64(acc3), d);
+    // `count` columns from constraint k on, all of them loaded first.
+    auto batch = [&](uint32_t k, uint32_t count) {
+      uint32_t v[U][R];
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u)
+        if (u < count) load_rows<R>(p + (uint64_t)(k + u) * stride, v[u]);
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u) {
+        if (u >= count) break;
+        const uint4 q = sco[k + u];
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+          const uint32_t w = v[u][j], cons = msub(w, madd(a[j], b[j]));
+          a[j] = b[j];
+          b[j] = mmul(w, w);
+          acc[j][0] += (uint64_t)q.x * cons; acc[j][1] += (uint64_t)q.y * cons;
+          acc[j][2] += (uint64_t)q.z * cons; acc[j][3] += (uint64_t)q.w * cons;
+          if (u % 3 == 2) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[j][c] = mfold64(acc[j][c]);
+          }
+        }
+      }
+    };
+    uint32_t k = 0;
+    for (; k + U <= n_cons; k += U) batch(k, U);
+    if (k < n_cons) batch(k, n_cons - k);
+    const uint32_t d = (row0 >> log_n) ? den1 : den0;  // the R rows share row >> log_n
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      uint32_t* o = out + (uint64_t)c * out_stride + row0;
+      if (R == 2) *reinterpret_cast<uint2*>(o) = make_uint2(mmul(mreduce64(acc[0][c]), d), mmul(mreduce64(acc[R - 1][c]), d));
+      else *o = mmul(mreduce64(acc[0][c]), d);
+    }
   }
 }
 
@@ -996,10 +1048,16 @@ cudaError_t wide_fib_trace(uint32_t log_n, uint32_t W, int kind, uint64_t seed, 
 cudaError_t wide_fib_composition(uint32_t log_n, uint32_t W, const uint32_t* eval, uint64_t stride,
                                  const QM31* coeffs_dev, uint32_t den_inv0, uint32_t den_inv1, uint32_t* out,
                                  uint64_t out_stride, cudaStream_t stream) {
-  const size_t smem = (size_t)(W - 2) * 16;
-  if ((2u << log_n) < MMA_ROWS) {
-    k_composition<<<grid_for(2ull << log_n, 256), 256, smem, stream>>>(log_n, W, eval, stride, coeffs_dev, den_inv0,
-                                                                       den_inv1, out, out_stride);
+  // Fewer rows than a warp's block of the tensor-core kernel, or so few columns that padding them to steps of eight
+  // costs it more than its products save (2^21 rows: 3 columns 17 us here, 32 there; 9: 35, 46; 14: 46, 47; 16: 54,
+  // 47; 17: 54, 60; 20: 60, 60; 24: 74, 60).
+  const bool few_rows = (2u << log_n) < MMA_ROWS;
+  if (few_rows || W < 16 || (W > 16 && W <= 20)) {
+    const bool pairs = ((reinterpret_cast<uintptr_t>(eval) | reinterpret_cast<uintptr_t>(out)) & 7) == 0 &&
+                       stride % 2 == 0 && out_stride % 2 == 0;
+    auto kernel = few_rows ? k_composition<1, 24> : pairs ? k_composition<2, 6> : k_composition<1, 6>;
+    kernel<<<grid_for(2ull << log_n, pairs ? 512 : 256), 256, (size_t)(W - 2) * 16, stream>>>(
+        log_n, W, eval, stride, coeffs_dev, den_inv0, den_inv1, out, out_stride);
     note_launch();
     return cudaGetLastError();
   }

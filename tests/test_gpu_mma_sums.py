@@ -1,6 +1,7 @@
 """The column sums on the tensor cores (composition, quotients) at the edges of their blocks: the
-smallest domains that take them and one below, column counts around a group of eight, columns and
-outputs that are not 16-byte aligned; against the definitions in Python integers."""
+smallest domains that take them and those below, column counts around a group of eight and around the
+narrow ones that the composition sums row by row, columns and outputs that are not 16-byte aligned;
+against the definitions in Python integers."""
 import numpy as np
 import pytest
 
@@ -28,7 +29,8 @@ def _words(t):
 
 
 @pytest.mark.parametrize("log_n,W,offset", [(3, 3, 0), (4, 9, 0), (5, 3, 0), (5, 8, 0), (6, 9, 0), (7, 16, 2), (6, 17, 3),
-                                            (14, 24, 0)])
+                                            (14, 24, 0), (1, 51, 3), (3, 26, 0), (4, 27, 1), (4, 100, 2), (6, 15, 0), (6, 14, 1),
+                                            (6, 16, 0), (7, 20, 2), (6, 20, 3), (6, 21, 0)])
 def test_composition(ctx, log_n, W, offset):
     rng = np.random.default_rng(10 * log_n + W)
     rows = 2 << log_n
