@@ -502,6 +502,10 @@ __global__ void k_oods_sum(const QM31* partial, uint32_t n_chunks, uint32_t n_co
 // ---------------------------------------------------------------------------
 constexpr uint32_t QUOT_MAX_ENTRIES = 1024;
 
+// One row per thread, for domains of fewer than 64 rows: few threads that wait for memory, so QUOT_U entries are
+// loaded before they are used (1024 columns on 16 rows: 260 us an entry at a time, 67 us now).
+constexpr uint32_t QUOT_U = 24;  // a multiple of three: the sums are folded after every third product
+
 __global__ void __launch_bounds__(256) k_quotients(PointTable pts, uint32_t log_size, uint32_t n_batches,
                                                    const QuotientBatchDev* batches,
                                                    const __grid_constant__ QuotientBatchDev one,
@@ -521,14 +525,24 @@ __global__ void __launch_bounds__(256) k_quotients(PointTable pts, uint32_t log_
     for (uint32_t b = 0; b < n_batches; ++b) {
       const QuotientBatchDev bt = batches[b];
       uint64_t a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-      for (uint32_t i = 0; i < bt.count; ++i) {
-        uint32_t e = bt.first + i;
-        uint32_t v = __ldg(col_ptrs[e] + row);
-        const uint32_t* q = sq + 4 * e;
-        a0 += (uint64_t)q[0] * v; a1 += (uint64_t)q[1] * v;
-        a2 += (uint64_t)q[2] * v; a3 += (uint64_t)q[3] * v;
-        if (i % 3 == 2) { a0 = mfold64(a0); a1 = mfold64(a1); a2 = mfold64(a2); a3 = mfold64(a3); }
-      }
+      // `count` entries from e on, all of their words loaded first.
+      auto take = [&](uint32_t e, uint32_t count) {
+        uint32_t v[QUOT_U];
+#pragma unroll
+        for (uint32_t u = 0; u < QUOT_U; ++u)
+          if (u < count) v[u] = __ldg(col_ptrs[e + u] + row);
+#pragma unroll
+        for (uint32_t u = 0; u < QUOT_U; ++u) {
+          if (u >= count) break;
+          const uint32_t* q = sq + 4 * (e + u);
+          a0 += (uint64_t)q[0] * v[u]; a1 += (uint64_t)q[1] * v[u];
+          a2 += (uint64_t)q[2] * v[u]; a3 += (uint64_t)q[3] * v[u];
+          if (u % 3 == 2) { a0 = mfold64(a0); a1 = mfold64(a1); a2 = mfold64(a2); a3 = mfold64(a3); }
+        }
+      };
+      uint32_t i = 0;
+      for (; i + QUOT_U <= bt.count; i += QUOT_U) take(bt.first + i, QUOT_U);
+      if (i < bt.count) take(bt.first + i, bt.count - i);
       QM31 num = qmake(mreduce64(a0), mreduce64(a1), mreduce64(a2), mreduce64(a3));
       num = qsub(num, qadd(qmulm(bt.sum_a, dp.y), bt.sum_b));
       CM31 prx = bt.point.x.c0, pry = bt.point.y.c0, pix = bt.point.x.c1, piy = bt.point.y.c1;

@@ -48,7 +48,8 @@ def test_composition(ctx, log_n, W, offset):
     assert np.array_equal(_words(out).reshape(4, rows), ref)
 
 
-@pytest.mark.parametrize("log,n,offset", [(5, 9, 0), (6, 1, 0), (6, 8, 0), (7, 13, 0), (6, 17, 1), (7, 24, 2)])
+@pytest.mark.parametrize("log,n,offset", [(5, 9, 0), (6, 1, 0), (6, 8, 0), (7, 13, 0), (6, 17, 1), (7, 24, 2), (2, 24, 0),
+                                          (3, 25, 0), (5, 49, 1), (5, 27, 2)])
 def test_quotients(ctx, log, n, offset):
     import torch
     rng = np.random.default_rng(10 * log + n)
