@@ -9,9 +9,10 @@
 // One thread per leaf: a warp reads 32 consecutive rows of a column as one
 // 128-byte transaction; the message schedule and state stay in registers.
 // Each CTA hashes 256 leaves and then folds the three node levels whose parents fill whole warps
-// (128, 64, 32) in shared memory, writing every level; a tree that fits one CTA is folded to its root there. The layers above are
-// folded by k_merkle_nodes, four levels per launch, while there are more than 2^12 children, and the
-// rest by one launch of k_merkle_top.
+// (128, 64, 32) in shared memory, writing every level; a tree that fits one CTA is folded to its root
+// there. The layers above are folded by k_merkle_nodes, four levels per launch, while there are more
+// than 2^9 children, and the rest by one CTA of k_merkle_top (the 2^12 first nodes of 2^15 leaves by a
+// cluster of eight).
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -31,7 +32,8 @@ constexpr uint32_t LEAF_THREADS = 256;  // leaves per CTA
 constexpr uint32_t LEAF_LEVELS = 8;     // a tree of up to 2^8 leaves folds in its leaf CTA
 constexpr uint32_t FULL_WARP_LEVELS = 3;  // levels whose parents fill whole warps (128, 64, 32)
 constexpr uint32_t NODE_THREADS = 256;  // parents per CTA at the first level
-constexpr uint32_t NODE_FOLD_LOG = 12;  // layers of up to 2^12 nodes fold in one launch (k_merkle_top)
+// The first nodes (2^12) of a tree of 2^15 leaves fold in one cluster launch (k_merkle_top).
+constexpr uint32_t CLUSTER_LOG = 12, CLUSTER_MAX_LOG = CLUSTER_LOG + FULL_WARP_LEVELS;
 
 struct Seeds { uint32_t leaf[8], node[8]; };
 
@@ -399,10 +401,9 @@ __device__ __forceinline__ uint32_t quad_fold(QuadBuffers& sm, const QuadLane& L
   return 0;
 }
 
-// The top of a tree, the layers above 2^child_log children (child_log <= 12), in one launch: one CTA up
-// to 2^9 children, above that a cluster of 2, 4 or 8 CTAs, each folding 512 children to one node;
-// every CTA sends its node to CTA 0's shared memory, which folds the last levels. 2^12 children took
-// 14.2 us in eight CTAs plus 5.5 us and a launch in one with one lane per hash; in CTAs of 512 threads 16.7 us, now 19-26 us.
+// The top of a tree, the layers above 2^child_log children, in one launch: one CTA up to 2^9 children,
+// above that a cluster of 2^(child_log - 9) <= 8 CTAs, each folding 512 children to one node; every CTA sends its node
+// to CTA 0's shared memory, which folds the last levels. merkle_finish says where a cluster is worth it.
 __global__ void __launch_bounds__(QUAD_THREADS, 3) k_merkle_top(uint8_t* layers, uint32_t max_log, uint32_t child_log,
                                                              Seeds seeds, uint32_t one) {
   __shared__ __align__(16) QuadBuffers sm;
@@ -697,9 +698,12 @@ static uint32_t leaf_levels(uint32_t log) { return log <= LEAF_LEVELS ? log : FU
 static cudaError_t merkle_finish(uint8_t* layers, uint32_t max_log, uint32_t child_log, cudaStream_t stream) {
   const Seeds& seeds = seeds_once();
   cudaError_t e = cudaSuccess;
-  // Large layers: four levels per launch, each CTA folding 512 children (every level's
-  // parents fill whole warps: 256, 128, 64, 32), until 2^9 .. 2^12 are left.
-  while (child_log > NODE_FOLD_LOG) {
+  // Four levels per launch, each CTA folding 512 children (every level's parents fill whole warps: 256, 128, 64,
+  // 32), until 2^6 .. 2^9 are left for one CTA. A cluster folds the last 2^12 at once where they are a small tree's
+  // first nodes: a call on 2^15 leaves takes 46 us, 47.4 with two launches. Above larger trees the cluster costs more
+  // than the launch it saves (2^18 leaves of 4 columns 72.2 against 66.6 us, 2^19 of 100 columns 233 against 226),
+  // and so it does on 2^10 and 2^11 (2^13 leaves 45.7, 42.0).
+  while (child_log > 9 && !(child_log == CLUSTER_LOG && max_log == CLUSTER_MAX_LOG)) {
     const uint32_t blocks = (uint32_t)((1ull << child_log) / (2 * NODE_THREADS));
     e = launch_chained(k_merkle_nodes, blocks, NODE_THREADS, 0, stream, layers, max_log, child_log, 4u, seeds, 1u);
     note_launch();

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 P = 2**31 - 1
 
 
-@pytest.mark.parametrize("log", [8, 9, 10, 11, 12, 13, 14, 15, 16])
+@pytest.mark.parametrize("log", [8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 18, 19])
 def test_every_layer(ctx, log):
     import torch
     cols = np.random.default_rng(log).integers(0, P, size=(3, 1 << log), dtype=np.uint32)
