@@ -28,9 +28,19 @@ constexpr int LU_THREADS = 256;
 constexpr int SCAN_PER_THREAD = 4;
 constexpr int SCAN_BLOCK = LU_THREADS * SCAN_PER_THREAD;  // positions per scan block
 
-// sum_j alphas[j] word_j - z, accumulated lazily per coordinate in 64 bits (folded every third product).
+// sum_j alphas[j] word_j - z. LAZY: accumulated per coordinate in 64 bits, folded every third product; else each
+// product is reduced (logup_interaction says where).
+template <bool LAZY>
 __device__ __forceinline__ QM31 use_denominator(const LogupParams& p, const LogupUse& u, uint64_t row) {
   const QM31 nz = qneg(p.z);
+  if (!LAZY) {
+    QM31 acc = nz;
+    for (uint32_t j = 0; j < u.n_words; ++j) {
+      const uint32_t w = u.words[j] ? u.words[j][row] : u.constants[j];
+      acc = qadd(acc, qmulm(p.alphas[j], w));
+    }
+    return acc;
+  }
   uint64_t a0 = nz.c0.a, a1 = nz.c0.b, a2 = nz.c1.a, a3 = nz.c1.b;
   for (uint32_t j = 0; j < u.n_words; ++j) {
     const uint32_t w = u.words[j] ? __ldg(u.words[j] + row) : u.constants[j];
@@ -48,13 +58,14 @@ __device__ __forceinline__ uint32_t use_numerator(const LogupUse& u, uint64_t ro
 }
 
 // Numerator and denominator of interaction column c at `row`.
+template <bool LAZY>
 __device__ __forceinline__ void column_fraction(const LogupParams& p, uint32_t c, uint64_t row, QM31& num,
                                                 QM31& den) {
   uint32_t u0 = c * p.batch;
-  QM31 da = use_denominator(p, p.uses[u0], row);
+  QM31 da = use_denominator<LAZY>(p, p.uses[u0], row);
   uint32_t ma = use_numerator(p.uses[u0], row);
   if (p.batch == 2 && u0 + 1 < p.n_uses) {
-    QM31 db = use_denominator(p, p.uses[u0 + 1], row);
+    QM31 db = use_denominator<LAZY>(p, p.uses[u0 + 1], row);
     uint32_t mb = use_numerator(p.uses[u0 + 1], row);
     num = qadd(qmulm(da, mb), qmulm(db, ma));
     den = qmul(da, db);
@@ -76,6 +87,7 @@ __device__ __forceinline__ void col_store(uint32_t* out, uint64_t stride, uint32
   b[3 * stride] = v.c1.b;
 }
 
+template <bool LAZY>
 __global__ void __launch_bounds__(LU_THREADS) k_logup_fractions(const __grid_constant__ LogupParams p, uint32_t* out,
                                                                 uint64_t stride, uint32_t* zero_flag) {
   uint64_t row = (uint64_t)blockIdx.x * LU_THREADS + threadIdx.x;
@@ -85,7 +97,7 @@ __global__ void __launch_bounds__(LU_THREADS) k_logup_fractions(const __grid_con
   QM31 suffix = qone();
   for (uint32_t c = n_cols; c-- > 0;) {
     QM31 num, den;
-    column_fraction(p, c, row, num, den);
+    column_fraction<LAZY>(p, c, row, num, den);
     col_store(out, stride, c, row, qmul(num, suffix));
     suffix = qmul(suffix, den);
   }
@@ -97,7 +109,7 @@ __global__ void __launch_bounds__(LU_THREADS) k_logup_fractions(const __grid_con
   QM31 running = qinv(suffix), acc = qzero();
   for (uint32_t c = 0; c < n_cols; ++c) {
     QM31 num, den;
-    column_fraction(p, c, row, num, den);
+    column_fraction<LAZY>(p, c, row, num, den);
     acc = qadd(acc, qmul(col_load(out, stride, c, row), running));
     col_store(out, stride, c, row, acc);
     running = qmul(running, den);
@@ -119,7 +131,7 @@ __global__ void __launch_bounds__(LU_THREADS) k_logup_fractions_reg(const __grid
   QM31 num[C], den[C], pre[C];
 #pragma unroll
   for (int c = 0; c < C; ++c) {
-    column_fraction(p, c, row, num[c], den[c]);
+    column_fraction<true>(p, c, row, num[c], den[c]);
     pre[c] = c == 0 ? den[0] : qmul(pre[c - 1], den[c]);
   }
   if (qiszero(pre[C - 1])) {
@@ -385,9 +397,16 @@ cudaError_t logup_interaction(const LogupParams& p, uint32_t* out, uint64_t out_
     return cudaErrorInvalidValue;
   const uint64_t rows = 1ull << p.log_rows;
   const uint32_t n_cols = logup_n_cols(p.n_uses, p.batch);
+  // Above the register kernels' four columns the denominators are formed twice, and reducing each product keeps the
+  // chain of a use shorter: sixteen uses of two words at 2^14 rows 25.1 us, lazily 26.6, and 385 against 394 at
+  // 2^20. Uses of many words over rows enough to hide the chain gain from fewer instructions instead: six of eight
+  // words at 2^20 rows 279 us, else 300 (at 2^16 29.1 against 27.7).
+  uint32_t max_words = 0;
+  for (uint32_t u = 0; u < p.n_uses; ++u) max_words = std::max(max_words, p.uses[u].n_words);
+  const bool lazy = p.log_rows >= 18 && max_words > 4;
   auto fractions = n_cols == 1 ? k_logup_fractions_reg<1> : n_cols == 2 ? k_logup_fractions_reg<2>
                  : n_cols == 3 ? k_logup_fractions_reg<3> : n_cols == LOGUP_REG_COLS ? k_logup_fractions_reg<LOGUP_REG_COLS>
-                               : k_logup_fractions;
+                 : lazy ? k_logup_fractions<true> : k_logup_fractions<false>;
   fractions<<<(unsigned)((rows + LU_THREADS - 1) / LU_THREADS), LU_THREADS, 0, stream>>>(p, out, out_stride, zero_flag);
   note_launch();
   uint32_t* last = out + 4ull * (n_cols - 1) * out_stride;

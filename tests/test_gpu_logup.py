@@ -170,6 +170,19 @@ def test_fractions_by_column_count(ctx, n_uses, batch, n_words):
     assert np.array_equal(got, ref) and np.array_equal(gc, rc)
 
 
+@pytest.mark.parametrize("n_words", [4, 5, 8])
+def test_many_rows_of_long_uses(ctx, n_words):
+    """2^18 rows and more than four words a use: the general kernel adds the products up unreduced."""
+    rng = np.random.default_rng(n_words)
+    cols = [rng.integers(0, P, size=1 << 18, dtype=np.uint32) for _ in range(n_words)]
+    for c in cols:
+        c[:4] = P - 1
+    uses = [dict(words=[cols[(u + j) % n_words] for j in range(n_words if u == 3 else 2)], negate=u == 1) for u in range(5)]
+    alphas = [[P - 1] * 4] + [rng.integers(0, P, size=4).tolist() for _ in range(n_words - 1)]
+    ref, rc, got, gc = _run_both(ctx, 18, uses, alphas, rng.integers(0, P, size=4).tolist(), 1, 1)
+    assert np.array_equal(got, ref) and np.array_equal(gc, rc)
+
+
 @pytest.mark.parametrize("log_rows,offset", [(10, 0), (10, 1), (11, 2), (12, 1)])
 def test_coset_scan_alignment(ctx, log_rows, offset):
     """The scan by whole sectors takes 16-byte aligned columns from 2^10 rows; others go row by row."""
