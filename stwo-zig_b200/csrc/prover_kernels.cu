@@ -724,8 +724,8 @@ __global__ void __launch_bounds__(MMA_THREADS, 4) k_quotients_mma(PointTable pts
 // completing on the stage's `full` mbarrier with the stage's byte count). A consumer warp waits on
 // `full`, reads its threads' two words of each column, and arrives on the stage's `empty` mbarrier;
 // the producer refills a stage once all eight consumer warps have arrived. The loads of the stages
-// ahead stay in flight while one is consumed, without the registers the register kernel's loads in
-// flight take, and the producer never holds the consumers at a block barrier. Items run batch by
+// ahead stay in flight while one is consumed without taking registers, and the producer never holds the
+// consumers at a block barrier. Items run batch by
 // batch (a batch's entries in groups of at most QB_GROUP); the last group of a batch adds the
 // batch's quotient. Each wait is bounded (about a second of the global timer): a side that runs out
 // sets QUOT_STATUS_TIMEOUT in *status and a shared abort flag that ends the other side's loop; the

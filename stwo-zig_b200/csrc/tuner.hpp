@@ -1,11 +1,11 @@
 // Launch-shape autotuner, process-wide and keyed by (op, log_size, n_cols).
 //
 // Some kernels come in variants that write the same bits but differ in speed with the shape: the
-// fused or generic FFT high pass, the Merkle leaf kernel built for 4, 5 or 6 CTAs per SM. The first call of a key runs every
-// variant of its op on that call's own inputs, timed with CUDA events on the call's stream (the
-// best of three interleaved runs each), and records the fastest; every later call of the key runs that variant.
-// An op whose outputs overwrite its inputs (an in-place transform) cannot be re-run and takes its
-// first variant untimed. Forcing a variant (tests, A/B runs) bypasses the table.
+// fused or generic FFT high pass, the Merkle leaf kernel built for 4, 5 or 6 CTAs per SM. The first
+// call of a key runs every variant of its op on that call's own inputs, timed with CUDA events on the
+// call's stream (the best of three interleaved runs each), and records the fastest; every later call
+// of the key runs that variant. An op whose outputs overwrite its inputs (an in-place transform, an
+// extension over its evaluations) cannot be re-run and takes its first variant untimed. Forcing a variant (tests, A/B runs) bypasses the table.
 #pragma once
 #include <cuda_runtime.h>
 

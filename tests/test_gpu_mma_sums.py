@@ -71,9 +71,11 @@ def test_quotients(ctx, log, n, offset):
         assert got[:, row].tolist() == list(V.qflat(V.qmulc(num, V.cinv(den)))), row
 
 
-@pytest.mark.parametrize("log,n", [(0, 3), (3, 2), (11, 5), (12, 1), (13, 33), (14, 600), (16, 160), (18, 38)])
+@pytest.mark.parametrize("log,n", [(0, 3), (3, 2), (11, 5), (12, 1), (13, 33), (14, 600), (16, 160), (18, 38), (16, 3000),
+                                   (17, 1500)])
 def test_openings(ctx, log, n):
-    """Below the tensor-core kernel's 2^12, with a chunk per warp and per CTA, several chunks a warp."""
+    """Below the tensor-core kernel's 2^12, with a chunk per CTA (n few) and per warp, and four chunks a warp in one and
+    two CTAs a column (the last two)."""
     import torch
     rng = np.random.default_rng(log)
     cols = rng.integers(0, P, size=(n, 1 << log), dtype=np.uint32)
@@ -84,3 +86,16 @@ def test_openings(ctx, log, n):
     got = _words(out).reshape(n, 4)
     for c in {0, n // 2, n - 1}:
         assert np.array_equal(got[c], oracle.eval_at_point(cols[c], px, py)), c
+
+
+def test_openings_of_more_chunks_than_the_factor_table(ctx):
+    """One CTA a column of 2^25 coefficients: 2048 chunks a warp, whose factors beyond the table's 1024 are multiplied
+    in. Every column is the same one (stride 0), as so many would not fit the device."""
+    import torch
+    log, n = 25, 2960
+    col = np.random.default_rng(log).integers(0, P, size=1 << log, dtype=np.uint32)
+    px, py = np.random.default_rng(log).integers(0, P, size=(2, 4)).tolist()
+    out = torch.empty(4 * n, dtype=torch.int32, device="cuda")
+    ctx.eval_at_point(_dev(col, 0), log, n, 0, px, py, out)
+    got = _words(out).reshape(n, 4)
+    assert (got == oracle.eval_at_point(col, px, py)).all()

@@ -1,8 +1,8 @@
-"""The DEEP quotient op's launch variants, above all the bulk-staged kernel (the fourth): a CTA streams
+"""The DEEP quotients' bulk-staged kernel (forced as variant 3; variants 0 to 2 are the tensor-core kernel): a CTA streams
 512-row chunks of its columns into a shared-memory ring with 1-D bulk async copies completing on
 mbarriers. Proofs through it equal the oracle's bytes (one batch of 24 to 1008 entries, entry counts
 that are not a multiple of the 8-column group, the XOR-lookup AIR's several batches), the op agrees
-with the register kernels, and its bounded waits, made to run out by a test hook (a stage whose
+with the tensor-core kernel, and its bounded waits, made to run out by a test hook (a stage whose
 copies are never issued), end the proof or the op with an error while the context stays usable.
 No GPU fault is involved: the hook only leaves a barrier phase incomplete."""
 import numpy as np
@@ -49,9 +49,9 @@ def test_xor_proofs_through_the_staged_kernel_equal_the_oracle(ctx, staged, log_
 
 
 @pytest.mark.parametrize("variant", [1, 2])
-def test_xor_proofs_through_the_other_quotient_variants_equal_the_oracle(ctx, variant):
-    """The XOR-lookup AIR's quotients come in several batches: the register variants with 3 and 9
-    loads in flight against the oracle's bytes."""
+def test_xor_proofs_under_the_other_forced_variants_equal_the_oracle(ctx, variant):
+    """Forced variants 1 and 2 change the leaf kernel and the high FFT pass of a proof; its quotients, in several
+    batches, are the tensor-core kernel's under both."""
     import stwo_b200 as sb
     o, g = _cfg("functional")
     try:
@@ -74,8 +74,8 @@ def _quotient_case(n_cols, log):
 
 
 @pytest.mark.parametrize("n_cols", [1, 8, 13, 108])
-def test_quotient_op_variants_equal_the_register_kernel(ctx, n_cols):
-    """Every quotient variant writes the first variant's words at the op level."""
+def test_staged_quotient_op_equals_the_tensor_core_kernel(ctx, n_cols):
+    """The staged kernel writes the tensor-core kernel's words at the op level, as variants 0 to 2 do."""
     import stwo_b200 as sb
     import torch
     log = 17

@@ -31,6 +31,19 @@ def test_fri_tail(ctx, log_n, last):
     assert got == oracle.prove_wide_fib(log_n, 5, o, trace_kind=1, trace_seed=log_n)
 
 
+def test_fri_tails_of_many_proofs_in_flight(ctx):
+    """Eight proofs' tails and tree tops beside other proofs' grinds: a cluster's CTAs start apart from one another,
+    and each has to read the channel's state before the first one moves it on."""
+    import stwo_b200 as sb
+    o = oracle.config("functional", pow_bits=22)
+    g = sb.PcsConfig(o.pow_bits, sb.FriConfig(o.log_blowup_factor, o.log_last_layer_degree_bound, o.n_queries))
+    requests = [{"statement": sb.Statement(12 + i % 3, 5), "config": g, "trace_kind": sb.TRACE_SEEDED, "trace_seed": 90 + i}
+                for i in range(24)]
+    want = [oracle.prove_wide_fib(12 + i % 3, 5, o, trace_kind=1, trace_seed=90 + i) for i in range(24)]
+    for _ in range(4):
+        assert ctx.prove_wide_fibonacci_batch(requests, max_in_flight=8) == want
+
+
 @pytest.mark.parametrize("bits", [3, 11, 16, 18, 20, 21, 22])
 def test_grind_round_shapes(ctx, bits):
     """Targets whose rounds have one nonce a thread, several, a full round's grid; the lowest nonce each time."""
