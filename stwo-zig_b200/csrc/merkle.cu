@@ -11,8 +11,8 @@
 // Each CTA hashes 256 leaves and then folds the three node levels whose parents fill whole warps
 // (128, 64, 32) in shared memory, writing every level; a tree that fits one CTA is folded to its root
 // there. The layers above are folded by k_merkle_nodes, four levels per launch, while there are more
-// than 2^9 children, and the rest by one CTA of k_merkle_top (the 2^12 first nodes of 2^15 leaves by a
-// cluster of eight).
+// than 2^9 children, and the rest by one CTA of k_merkle_top, or by a cluster of them where that is
+// the shorter way (merkle_finish).
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -32,8 +32,8 @@ constexpr uint32_t LEAF_THREADS = 256;  // leaves per CTA
 constexpr uint32_t LEAF_LEVELS = 8;     // a tree of up to 2^8 leaves folds in its leaf CTA
 constexpr uint32_t FULL_WARP_LEVELS = 3;  // levels whose parents fill whole warps (128, 64, 32)
 constexpr uint32_t NODE_THREADS = 256;  // parents per CTA at the first level
-// The first nodes (2^12) of a tree of 2^15 leaves fold in one cluster launch (k_merkle_top).
-constexpr uint32_t CLUSTER_LOG = 12, CLUSTER_MAX_LOG = CLUSTER_LOG + FULL_WARP_LEVELS;
+// Layers of 2^10 .. 2^12 nodes fold in one cluster launch (k_merkle_top) in trees of 2^15 .. 2^17 leaves.
+constexpr uint32_t CLUSTER_LOG = 12, CLUSTER_MIN = 15, CLUSTER_MAX = 17;
 
 struct Seeds { uint32_t leaf[8], node[8]; };
 
@@ -699,11 +699,12 @@ static cudaError_t merkle_finish(uint8_t* layers, uint32_t max_log, uint32_t chi
   const Seeds& seeds = seeds_once();
   cudaError_t e = cudaSuccess;
   // Four levels per launch, each CTA folding 512 children (every level's parents fill whole warps: 256, 128, 64,
-  // 32), until 2^6 .. 2^9 are left for one CTA. A cluster folds the last 2^12 at once where they are a small tree's
-  // first nodes: a call on 2^15 leaves takes 46 us, 47.4 with two launches. Above larger trees the cluster costs more
-  // than the launch it saves (2^18 leaves of 4 columns 72.2 against 66.6 us, 2^19 of 100 columns 233 against 226),
-  // and so it does on 2^10 and 2^11 (2^13 leaves 45.7, 42.0).
-  while (child_log > 9 && !(child_log == CLUSTER_LOG && max_log == CLUSTER_MAX_LOG)) {
+  // 32), until 2^6 .. 2^9 are left for one CTA. In trees of 2^15 and 2^17 leaves a cluster folds the last 2^12 and
+  // 2^10 at once, which saves a launch (a fold into 2^17 values 61.2 us, 63.0 with two launches). In smaller ones its
+  // CTAs are no faster than the launch they save (2^13 leaves of 4 columns 45.5 us, 40.5 with two launches; 2^14 of
+  // 100 columns 58.2, 53.7), and above larger ones it costs more (2^18 leaves of 4 columns 72.4, 65.7; 2^19 of 100
+  // columns 234, 225).
+  while (child_log > CLUSTER_LOG || (child_log > 9 && (max_log < CLUSTER_MIN || max_log > CLUSTER_MAX))) {
     const uint32_t blocks = (uint32_t)((1ull << child_log) / (2 * NODE_THREADS));
     e = launch_chained(k_merkle_nodes, blocks, NODE_THREADS, 0, stream, layers, max_log, child_log, 4u, seeds, 1u);
     note_launch();
