@@ -31,6 +31,35 @@ def test_fri_tail(ctx, log_n, last):
     assert got == oracle.prove_wide_fib(log_n, 5, o, trace_kind=1, trace_seed=log_n)
 
 
+def test_roots_read_by_more_threads_than_slots(ctx):
+    """Roots come back through page-locked slots, and directly where every slot is taken: 48 threads on streams of
+    their own, each with its own columns."""
+    import threading
+    import torch
+    logs = [6 + i % 7 for i in range(48)]
+    cols = [np.random.default_rng(i).integers(0, P, size=(2, 1 << log), dtype=np.uint32) for i, log in enumerate(logs)]
+    want = [oracle.merkle_root(list(c)) for c in cols]
+    dev = [torch.from_numpy(c.view(np.int32)).cuda() for c in cols]
+    torch.cuda.synchronize()
+    wrong, start = [], threading.Barrier(48)
+
+    def work(i):
+        stream = torch.cuda.Stream()
+        layers = torch.empty(((2 << logs[i]) - 1) * 32, dtype=torch.uint8, device="cuda")
+        start.wait()
+        for _ in range(50):
+            if ctx.merkle_commit(dev[i], logs[i], 2, layers, stream=stream) != want[i]:
+                wrong.append(i)
+        stream.synchronize()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(48)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+
+
 def test_fri_tails_of_many_proofs_in_flight(ctx):
     """Eight proofs' tails and tree tops beside other proofs' grinds: a cluster's CTAs start apart from one another,
     and each has to read the channel's state before the first one moves it on."""
