@@ -605,7 +605,7 @@ __global__ void __launch_bounds__(1 << R, R <= 8 ? (1024 >> R) : 1) k_fft_high16
 // or the buffers overlap. Bound by launch and exchange latency. The generic passes (a block pass of 2^11 words
 // and a pass over 8 adjacent words of every block, two layers per shared-memory round trip) took, for
 // 100 columns of 2^12 -> 2^13, 10.7 + 74.9 + 10.2 us, and for 37 of 2^13 -> 2^15, 9.8 + 39.9 + 12.2 us; now 9.9 and
-// 11.3 us.
+// 11.7 us.
 struct SmallParams {
   const uint32_t* src; uint64_t ss;
   int do_inverse; TwiddleView itv; uint32_t scale; uint32_t* coef; uint64_t cs;

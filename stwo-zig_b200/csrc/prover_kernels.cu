@@ -595,8 +595,8 @@ __device__ __forceinline__ void quot_batch_finish(const QuotientBatchDev& bt, co
 // with zero coefficients. Lane t inverts the denominators of tile t's two rows, whose points are
 // conjugates, with one inversion, and the four lanes exchange them. ALIGNED: columns and output 16-byte aligned, with strides of a multiple of four words.
 //
-// Bound by HBM: 2^21 rows x 108 columns 168 us, 5.6 TB/s (the lazily accumulating register
-// kernel, ten instructions per word, 265 us; the bulk-staged one 258 us).
+// Bound by HBM: 2^21 rows x 108 columns 162 us, 5.8 TB/s, and 175 us where the kernel looks at the pointers (64-bit
+// multiply-adds, ten instructions per word, 265 us; the bulk-staged kernel 258 us).
 template <bool ALIGNED>
 __device__ __forceinline__ void quotients_mma_rows(const PointTable& pts, uint32_t log_size, uint32_t n_batches,
                                                    const QuotientBatchDev* batches, uint4* qmma, const uint32_t* sq,
